@@ -22,7 +22,8 @@ struct ElemConsts {
 };
 
 // local node i <-> q = ox<<2 | oy<<1 | oz   (het.cu:261-264)
-__device__ __constant__ int kQofLocal[8] = {0, 4, 6, 2, 1, 5, 7, 3};
+// (a function of constants, so that indexing by it keeps v[] in registers)
+__host__ __device__ constexpr int q_of_local(int i) { return (0x37512640u >> (4 * i)) & 7; }
 // canonical node sum: the corner q of each contributing element, in order
 __device__ __constant__ int kSumOrder[8] = {4, 7, 6, 5, 0, 3, 2, 1};
 
@@ -80,7 +81,7 @@ __device__ __forceinline__ void elem_wht(double* v, double rhoc, double dk, cons
 __device__ __forceinline__ void elem_fast(double* v, double rhoc, double dk, const ElemConsts& c) {
     double xl[8], yl[8];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) xl[i] = v[kQofLocal[i]];
+    for (int i = 0; i < 8; ++i) xl[i] = v[q_of_local(i)];
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
         double acc = 0.0;
@@ -92,7 +93,7 @@ __device__ __forceinline__ void elem_fast(double* v, double rhoc, double dk, con
         yl[i] = acc;
     }
 #pragma unroll
-    for (int i = 0; i < 8; ++i) v[kQofLocal[i]] = yl[i];
+    for (int i = 0; i < 8; ++i) v[q_of_local(i)] = yl[i];
 }
 
 // het.cu:310-338 with the multiply-adds made explicit
@@ -103,7 +104,7 @@ __device__ __forceinline__ void elem_gauss(double* v, double rhoc, double ke, do
     const double* gz = c.gtab + 192;
     double xl[8], yl[8];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) { xl[i] = v[kQofLocal[i]]; yl[i] = 0.0; }
+    for (int i = 0; i < 8; ++i) { xl[i] = v[q_of_local(i)]; yl[i] = 0.0; }
     for (int g = 0; g < 8; ++g) {
         for (int i = 0; i < 8; ++i) {
             double Mx = 0.0, Kx = 0.0;
@@ -120,7 +121,7 @@ __device__ __forceinline__ void elem_gauss(double* v, double rhoc, double ke, do
         }
     }
 #pragma unroll
-    for (int i = 0; i < 8; ++i) v[kQofLocal[i]] = yl[i];
+    for (int i = 0; i < 8; ++i) v[q_of_local(i)] = yl[i];
 }
 
 template <int FORM>
@@ -339,9 +340,19 @@ struct __align__(16) SlabSmem {
 };
 constexpr size_t kSlabSmem = sizeof(SlabSmem);
 
+// A load of a vector: read-only for the kernel's whole life (the non-coherent
+// path), or, with COH, written by other CTAs of the same launch before a grid
+// barrier (through the L2, past a possibly stale L1 line).
+template <bool COH, typename V>
+__device__ __forceinline__ V ld_vec(const V* p) {
+    if constexpr (COH) return __ldcg(p);
+    else return __ldg(p);
+}
+
 // MODE 0: input x as given; 1: PCG loop, p = z; 2: PCG loop, p = z + beta p_{k-1}.
 // FI false: no fault is armed for this launch (the per-node fault tests compile out).
-template <int FORM, int MODE, bool FI = true>
+// COH: the input vectors are written inside this launch (ld_vec).
+template <int FORM, int MODE, bool FI = true, bool COH = false>
 __device__ __forceinline__ void slab_march(const ApplyArgs& a, SlabSmem& S, const SlabTile& T, const SlabPos& G,
                                            const double* src_a, const double* src_b, double beta, double* pout,
                                            bool loop, bool d1, bool rhs, int fi_p, int fi_ap, int fi_r, int fi_bit,
@@ -364,8 +375,8 @@ __device__ __forceinline__ void slab_march(const ApplyArgs& a, SlabSmem& S, cons
         for (int k = 0; k < SK; ++k) {
             const bool v = pv && sp_valid(fl, k);
             const unsigned n = base + (unsigned)G.noff[k];
-            ra[k] = v ? __ldg(src_a + n) : 0.0;
-            if (TWO) rb[k] = v ? __ldg(src_b + n) : 0.0;
+            ra[k] = v ? ld_vec<COH>(src_a + n) : 0.0;
+            if (TWO) rb[k] = v ? ld_vec<COH>(src_b + n) : 0.0;
         }
     };
     auto form = [&](int px, double (&p)[SK]) {
@@ -611,12 +622,101 @@ __device__ __forceinline__ void update_scalars(const UpdateArgs& a, const double
     }
 }
 
-// PCG vector update on the flat partition: each thread updates its KF
-// consecutive nodes (KF / 2 aligned 128-bit loads and stores per vector), in
-// order.  In the loop it first finishes the operator's reductions: every CTA
-// sums p.Ap over the tile partials in the canonical order (so alpha = rho /
-// p.Ap is the same bits everywhere), and CTA 0 records p.Ap, alpha, the D1
-// checksum and a breakdown.
+// One step of the vector update: what every flat block of it shares.
+struct UpdStep {
+    bool pre, xupd;                 // prologue; the solution update of two iterations runs
+    double alpha, alpha_prev;
+    const double* p;                // p_k and p_{k-1}
+    const double* p_prev;
+    int fi_r, fi_bit;               // armed flip of r at fi_idx
+    long long fi_idx;
+};
+
+// The update of U flat blocks at once (U > 1: of U different runs, so that
+// their loads are in flight together): each thread takes its KF consecutive
+// nodes of each block (KF / 2 aligned 128-bit loads and stores per vector), in
+// order, and carries on its run's sums in part (PRE: b.b, r.z, r.r; LOOP: r.r,
+// r.z).  A block index of nflat or more is no block.
+template <int U, bool COH>
+__device__ __forceinline__ void upd_blocks(const UpdateArgs& a, const UpdStep& s, const long long (&blk)[U],
+                                           double (&part)[U][3]) {
+    static_assert(KF == 2, "one pair of nodes per thread and block");
+    const int tid = threadIdx.x;
+    long long m0[U];
+    int cnt[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+        m0[u] = (blk[u] * RT + tid) * KF;
+        cnt[u] = (blk[u] >= a.nflat) ? 0 : (m0[u] + 1 < a.Nn) ? 2 : (m0[u] < a.Nn ? 1 : 0);
+    }
+    auto ld = [&](const double* base, double (&v)[U][KF]) {
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            if (cnt[u] == 2) {
+                const double2 t = ld_vec<COH>(reinterpret_cast<const double2*>(base + m0[u]));
+                v[u][0] = t.x; v[u][1] = t.y;
+            } else { v[u][0] = cnt[u] ? ld_vec<COH>(base + m0[u]) : 0.0; v[u][1] = 0.0; }
+        }
+    };
+    auto stv = [&](double* base, const double (&v)[U][KF]) {
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            if (cnt[u] == 2) *reinterpret_cast<double2*>(base + m0[u]) = make_double2(v[u][0], v[u][1]);
+            else if (cnt[u] == 1) base[m0[u]] = v[u][0];
+        }
+    };
+    if (s.pre) {
+        double bb[U][KF], qq[U][KF], dd[U][KF];
+        ld(a.b, bb); ld(a.Ap, qq); ld(a.d, dd);
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+#pragma unroll
+            for (int k = 0; k < KF; ++k) {
+                if (k >= cnt[u]) continue;
+                const double r_ = dfma(-1.0, qq[u][k], bb[u][k]);
+                const double z_ = __ddiv_rn(r_, dd[u][k]);
+                part[u][0] = dfma(bb[u][k], bb[u][k], part[u][0]);
+                part[u][1] = dfma(r_, z_, part[u][1]);
+                part[u][2] = dfma(r_, r_, part[u][2]);
+                qq[u][k] = r_; dd[u][k] = z_;
+            }
+        stv(a.r, qq); stv(a.z, dd);
+        return;
+    }
+    double qq[U][KF], rr[U][KF], dd[U][KF];
+    ld(a.Ap, qq); ld(a.r, rr); ld(a.d, dd);
+    if (s.xupd) {
+        // x += alpha_{k-1} p_{k-1}, then x += alpha_k p_k: the same two
+        // multiply-adds, in the same order, as one update per iteration
+        double xx[U][KF], pp[U][KF], po[U][KF];
+        ld(a.x, xx); ld(s.p_prev, po); ld(s.p, pp);
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+#pragma unroll
+            for (int k = 0; k < KF; ++k)
+                if (k < cnt[u]) xx[u][k] = dfma(s.alpha, pp[u][k], dfma(s.alpha_prev, po[u][k], xx[u][k]));
+        stv(a.x, xx);
+    }
+    const double nalpha = -s.alpha;
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+#pragma unroll
+        for (int k = 0; k < KF; ++k) {
+            if (k >= cnt[u]) continue;
+            double rk = dfma(nalpha, qq[u][k], rr[u][k]);
+            if (s.fi_r && m0[u] + k == s.fi_idx) rk = flipbit(rk, s.fi_bit);
+            rr[u][k] = rk;
+            dd[u][k] = __ddiv_rn(rk, dd[u][k]);          // z
+            part[u][0] = dfma(rk, rk, part[u][0]);
+            part[u][1] = dfma(rk, dd[u][k], part[u][1]);
+        }
+    stv(a.r, rr); stv(a.z, dd);
+}
+
+// PCG vector update on the flat partition.  In the loop it first finishes the
+// operator's reductions: every CTA sums p.Ap over the tile partials in the
+// canonical order (so alpha = rho / p.Ap is the same bits everywhere), and
+// CTA 0 records p.Ap, alpha, the D1 checksum and a breakdown.
 //
 // It also finishes its own reductions, in the RUN order: CTA c of the
 // G = min(nflat, UPD_SLOTS) CTAs takes the flat blocks c, c+G, c+2G, ..., each
@@ -629,8 +729,6 @@ __device__ __forceinline__ void update_scalars(const UpdateArgs& a, const double
 constexpr int kUpdateCtasPerSm = 5;
 static_assert(UPD_SLOTS == 148 * kUpdateCtasPerSm, "one resident wave of update CTAs on 148 SMs");
 __global__ void __launch_bounds__(RT, kUpdateCtasPerSm) k_update(UpdateArgs a) {
-    static_assert(KF % 2 == 0, "pairs of nodes per thread");
-    constexpr int NC = KF / 2;
     __shared__ double sh[MAXQ][8];
     __shared__ double s_pAp;
     __shared__ unsigned s_last;
@@ -685,84 +783,23 @@ __global__ void __launch_bounds__(RT, kUpdateCtasPerSm) k_update(UpdateArgs a) {
         if (fabs(pAp) < 1e-30) return;          // breakdown: the reference stops before the update
         alpha = __ddiv_rn(st->rho, pAp);
     }
-    const double nalpha = -alpha;
     // x += alpha p runs at odd iterations, for the previous iteration and this
     // one (the previous p is still in the other buffer, its alpha in alpha_hist)
-    const bool xupd = !pre && (iter & 1);
-    const double* p_prev = (iter & 1) ? a.pbuf0 : a.pbuf1;
-    const double alpha_prev = xupd ? st->alpha_hist[(iter - 1) & 1] : 0.0;
-    // one flat block: its 3 partials (PRE: bb, rz, rr   LOOP: rr, rz, -) into part
-    auto block = [&](long long blk, double* part) {
-        const long long m0 = (blk * RT + tid) * KF;
-        int cnt[NC];
-#pragma unroll
-        for (int c = 0; c < NC; ++c) {
-            const long long m = m0 + 2 * c;
-            cnt[c] = (blk >= a.nflat) ? 0 : (m + 1 < a.Nn) ? 2 : (m < a.Nn ? 1 : 0);
-        }
-        auto ld = [&](const double* base, double (&v)[KF]) {
-#pragma unroll
-            for (int c = 0; c < NC; ++c) {
-                const long long m = m0 + 2 * c;
-                if (cnt[c] == 2) { const double2 t = __ldg(reinterpret_cast<const double2*>(base + m)); v[2 * c] = t.x; v[2 * c + 1] = t.y; }
-                else { v[2 * c] = cnt[c] ? __ldg(base + m) : 0.0; v[2 * c + 1] = 0.0; }
-            }
-        };
-        auto stv = [&](double* base, const double (&v)[KF]) {
-#pragma unroll
-            for (int c = 0; c < NC; ++c) {
-                const long long m = m0 + 2 * c;
-                if (cnt[c] == 2) *reinterpret_cast<double2*>(base + m) = make_double2(v[2 * c], v[2 * c + 1]);
-                else if (cnt[c] == 1) base[m] = v[2 * c];
-            }
-        };
-        auto has = [&](int k) { return k % 2 < cnt[k / 2]; };
-        if (pre) {
-            double bb[KF], qq[KF], dd[KF], r_[KF], z_[KF];
-            ld(a.b, bb); ld(a.Ap, qq); ld(a.d, dd);
-#pragma unroll
-            for (int k = 0; k < KF; ++k) {
-                r_[k] = 0.0; z_[k] = 0.0;
-                if (!has(k)) continue;
-                r_[k] = dfma(-1.0, qq[k], bb[k]);
-                z_[k] = __ddiv_rn(r_[k], dd[k]);
-                part[0] = dfma(bb[k], bb[k], part[0]);
-                part[1] = dfma(r_[k], z_[k], part[1]);
-                part[2] = dfma(r_[k], r_[k], part[2]);
-            }
-            stv(a.r, r_); stv(a.z, z_);
-        } else {
-            double qq[KF], rr[KF], dd[KF];
-            ld(a.Ap, qq); ld(a.r, rr); ld(a.d, dd);
-            if (xupd) {
-                // x += alpha_{k-1} p_{k-1}, then x += alpha_k p_k: the same two
-                // multiply-adds, in the same order, as one update per iteration
-                double xx[KF], pp[KF], po[KF];
-                ld(a.x, xx); ld(p_prev, po); ld(p, pp);
-#pragma unroll
-                for (int k = 0; k < KF; ++k)
-                    if (has(k)) xx[k] = dfma(alpha, pp[k], dfma(alpha_prev, po[k], xx[k]));
-                stv(a.x, xx);
-            }
-#pragma unroll
-            for (int k = 0; k < KF; ++k) {
-                if (!has(k)) continue;
-                double rk = dfma(nalpha, qq[k], rr[k]);
-                if (fi_r && m0 + k == fi_idx) rk = flipbit(rk, fi_bit);
-                rr[k] = rk;
-                dd[k] = __ddiv_rn(rk, dd[k]);          // z
-                part[0] = dfma(rk, rk, part[0]);
-                part[1] = dfma(rk, dd[k], part[1]);
-            }
-            stv(a.r, rr); stv(a.z, dd);
-        }
-    };
+    UpdStep us{};
+    us.pre = pre;
+    us.xupd = !pre && (iter & 1);
+    us.alpha = alpha;
+    us.alpha_prev = us.xupd ? st->alpha_hist[(iter - 1) & 1] : 0.0;
+    us.p = p;
+    us.p_prev = (iter & 1) ? a.pbuf0 : a.pbuf1;
+    us.fi_r = fi_r; us.fi_bit = fi_bit; us.fi_idx = fi_idx;
     // run blockIdx.x of the RUN order: flat blocks c, c+G, ...; each thread
     // carries one sum through its nodes of all the run's blocks, and the run
     // takes one block tree at the end
     const int G = gridDim.x, c = blockIdx.x;
-    double part[3] = {0.0, 0.0, 0.0};
-    for (int blk = c; blk < a.nflat; blk += G) block(blk, part);
+    double rp[1][3] = {{0.0, 0.0, 0.0}};
+    for (int blk = c; blk < a.nflat; blk += G) upd_blocks<1, false>(a, us, {blk}, rp);
+    double (&part)[3] = rp[0];
     cta_tree_sum<3>(part, sh);
     if (tid == 0) {
 #pragma unroll
@@ -1137,7 +1174,9 @@ struct StepCtl {
     int flipG, pad;
     long long gidx;
 };
-__global__ void k_step_begin(DevState* st, StepCtl c, double* T) {
+__global__ void k_step_begin(DevState* st, StepCtl c, double* T, unsigned* count) {
+    st->stuck = 0;
+    count[0] = count[32] = 0u;              // the cooperative solve's gates
     st->fi_armR = c.armR; st->fi_vec = c.vec; st->fi_iter = c.iter; st->fi_bit = c.bit;
     st->fi_elem = c.elem; st->fi_idx = c.idx;
     st->d1_step = 0.0;
@@ -1146,7 +1185,7 @@ __global__ void k_step_begin(DevState* st, StepCtl c, double* T) {
 __global__ void k_disarm_R(DevState* st) { st->fi_armR = 0; }
 __global__ void k_step_end(DevState* st, int* iters_out, double* d1_out) {
     st->fi_armR = 0; st->fi_vec = 0;
-    *iters_out = st->result;
+    *iters_out = st->stuck ? -1 : st->result;
     *d1_out = st->d1_step;
 }
 __global__ void k_d2_finish(const double* red, double* d2_out) {

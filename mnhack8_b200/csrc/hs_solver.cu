@@ -14,6 +14,7 @@
 #include "../../include/heat_b200.h"
 #include "hs_host.h"
 #include "hs_kernels.cuh"
+#include "hs_pcg.cuh"
 
 using namespace hs;
 
@@ -87,7 +88,10 @@ struct hs_solver {
     DevBuf<double> partials;            // operator tiles (and the standalone reductions)
     DevBuf<double> upart;               // PCG vector update: run sums (RUN order)
     int n_sm = 148;
-    DevBuf<unsigned> ticket;
+    DevBuf<unsigned> ticket;            // [0] last-CTA tickets; [64], [96] gates of the cooperative solve
+    int coop_grid = 0;                  // CTAs of the cooperative solve (k_pcg); 0: the graph's while loop instead
+    XWord* xwords = nullptr;            // its exchange words (in upart)
+    unsigned pcg_launches = 0;
     DevBuf<DevState> st;
     DevBuf<double> red;                 // standalone reduction outputs
     DevBuf<unsigned long long> sp;      // spread: [gmax bits, count]
@@ -203,19 +207,25 @@ void launch_atomic(hs_solver* h, const AtomArgs& a) {
     }
 }
 
+ApplyArgs colored_args(hs_solver* h, int role, const double* x, double* y, double dt_eff, bool d1, const double* w,
+                       const double* F, double dtF) {
+    ApplyArgs a{};
+    a.part = h->part;
+    a.N = h->N; a.role = role; a.dt_eff = dt_eff;
+    a.x = x; a.z = h->z.p; a.pbuf0 = h->p0.p; a.pbuf1 = h->p1.p;
+    a.y = y; a.coef = h->coef.p; a.w = w; a.F = F; a.dtF = dtF;
+    a.d1 = d1 ? 1 : 0;
+    a.partials = h->partials.p; a.st = h->st.p; a.ec = h->ec;
+    return a;
+}
+
 // Projected operator application y = A x (or the LOOP form p = z + beta p,
 // Ap = A p).  Colored: one fused kernel.  Atomic: zero, element scatter with
 // atomics, then projection + partials on the canonical partition.
 void apply_projected(hs_solver* h, int role, const double* x, double* y, double dt_eff, bool d1,
                      const double* w, const double* F, double dtF, bool pdl = false) {
     if (h->opt.scatter == HS_SCATTER_COLORED) {
-        ApplyArgs a{};
-        a.part = h->part;
-        a.N = h->N; a.role = role; a.dt_eff = dt_eff;
-        a.x = x; a.z = h->z.p; a.pbuf0 = h->p0.p; a.pbuf1 = h->p1.p;
-        a.y = y; a.coef = h->coef.p; a.w = w; a.F = F; a.dtF = dtF;
-        a.d1 = d1 ? 1 : 0;
-        a.partials = h->partials.p; a.st = h->st.p; a.ec = h->ec;
+        const ApplyArgs a = colored_args(h, role, x, y, dt_eff, d1, w, F, dtF);
         launch_colored(h, a, pdl);
         // the loop role's reductions are finished by the vector update (k_update)
         if (role != ROLE_LOOP && d1) {
@@ -245,15 +255,20 @@ void apply_projected(hs_solver* h, int role, const double* x, double* y, double 
     }
 }
 
-void launch_update(hs_solver* h, int role, bool use_cond, cudaGraphConditionalHandle cond = 0, bool pdl = false) {
+UpdateArgs update_args(hs_solver* h, int role) {
     UpdateArgs u{};
     u.Nn = h->Nn; u.nflat = h->part.nflat; u.role = role; u.x = h->T.p; u.b = h->b.p; u.r = h->r.p; u.z = h->z.p; u.Ap = h->Ap.p;
     u.d = h->diag.p; u.pbuf0 = h->p0.p; u.pbuf1 = h->p1.p; u.partials = h->upart.p; u.ticket = h->ticket.p;
-    u.st = h->st.p; u.cond = cond; u.use_cond = 0;
+    u.st = h->st.p;
     u.d1 = h->opt.detect != 0; u.apart = h->partials.p; u.nblk = h->part.nblk;
+    return u;
+}
+int update_runs(const hs_solver* h) { return (int)std::min<long long>(h->part.nflat, UPD_SLOTS); }
+void launch_update(hs_solver* h, int role, bool use_cond, cudaGraphConditionalHandle cond = 0, bool pdl = false) {
+    UpdateArgs u = update_args(h, role);
     u.cond = cond; u.use_cond = use_cond ? 1 : 0;
     // one CTA per run of the RUN order (one resident wave on B200)
-    launch_k(pdl, k_update, (int)std::min<long long>(h->part.nflat, UPD_SLOTS), RT, 0, h->s, u);
+    launch_k(pdl, k_update, update_runs(h), RT, 0, h->s, u);
 }
 
 // the solution update the loop still owes (x += alpha p of an even last iteration)
@@ -278,7 +293,8 @@ void enqueue_pcg_prologue(hs_solver* h, bool with_rhs) {
     launch_update(h, UPD_PRE, false);
 }
 
-// HS_GRAPH=0 in the environment launches the PCG loop directly from the host
+// The PCG loop as launches (grids the cooperative solve does not take, and the
+// atomic scatter).  HS_GRAPH=0 in the environment launches it directly from the host
 // (chunks of iterations, the device "done" flag read back between chunks)
 // instead of through the graph's while node: profilers cannot attribute
 // kernels that run inside a conditional graph node.
@@ -304,13 +320,82 @@ bool graphs_enabled() {
     return v == 1;
 }
 
+// ---- the cooperative solve -----------------------------------------------------
+template <int FORM>
+const void* pcg_kernel_form(int nk, bool runs) {
+    if (runs) return (const void*)k_pcg<FORM, 4, kPcgRuns>;
+    return nk <= 1 ? (const void*)k_pcg<FORM, 1, 1> : nk <= 2 ? (const void*)k_pcg<FORM, 2, 1> : (const void*)k_pcg<FORM, 4, 1>;
+}
+// the instantiation for a tile plane of Rw x Cw positions (ST per position of a
+// thread); runs: some CTA has more than one run
+const void* pcg_kernel(const hs_solver* h, bool runs) {
+    const int nk = (h->part.Rw * h->part.Cw + ST - 1) / ST;
+    switch (h->opt.kernel) {
+        case HS_KERNEL_WHT: return pcg_kernel_form<FORM_WHT>(nk, runs);
+        case HS_KERNEL_GAUSS: return pcg_kernel_form<FORM_GAUSS>(nk, runs);
+        default: return pcg_kernel_form<FORM_FAST>(nk, runs);
+    }
+}
+// CTAs of the cooperative solve: one per tile and per run (or per kPcgRuns runs)
+// where they are all resident at once; else 0 (the graph's while loop)
+hs_status set_coop_grid(hs_solver* h, int dev) {
+    h->coop_grid = 0;
+    if (h->opt.scatter != HS_SCATTER_COLORED || !graphs_enabled() || pdl_enabled()) return HS_OK;
+    // a run is one flat block up to N = 88; the waits take at most 2 RT tiles
+    if (h->part.nflat > UPD_SLOTS || h->part.nblk > 2 * RT) return HS_OK;
+    const size_t smem = pcg_smem(h->part.CX);
+    int can = 0, most = 0;
+    HS_CUDA(cudaDeviceGetAttribute(&can, cudaDevAttrCooperativeLaunch, dev));
+    HS_CUDA(cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+    if (!can || smem + 4096 > (size_t)most) return HS_OK;
+    for (const bool runs : {false, true}) {
+        const long long nf = h->part.nflat;
+        const long long grid = std::max(h->part.ntiles, runs ? (nf + kPcgRuns - 1) / kPcgRuns : nf);
+        int per_sm = 0;
+        const void* k = pcg_kernel(h, runs);
+        HS_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        HS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, ST, smem));
+        if ((long long)per_sm * h->n_sm < grid) continue;
+        h->coop_grid = (int)grid;
+        break;
+    }
+    return HS_OK;
+}
+hs_status launch_pcg(hs_solver* h, bool with_rhs) {
+    PcgArgs a{};
+    a.part = h->part;
+    a.dt = h->opt.dt; a.dtF = h->opt.dt;
+    a.coef = h->coef.p; a.wM = h->wM.p; a.wA = h->wA.p;
+    a.F = (!h->opt.verify && !h->opt.no_source && h->has_F) ? h->F.p : nullptr;
+    a.d = h->diag.p; a.x = h->T.p; a.b = h->b.p; a.r = h->r.p; a.z = h->z.p; a.Ap = h->Ap.p; a.pbuf0 = h->p0.p; a.pbuf1 = h->p1.p;
+    a.xa = h->xwords; a.xr = h->xwords + 2 * h->part.nblk;
+    a.dparts = h->partials.p;
+    a.count = h->ticket.p + 64;
+    a.tag = (unsigned long long)++h->pcg_launches << 32;     // tags of different launches never meet
+    a.st = h->st.p;
+    a.with_rhs = with_rhs ? 1 : 0;
+    a.nruns = update_runs(h);
+    a.d1 = h->opt.detect != 0;
+    a.ec = h->ec;
+    void* args[] = {&a};
+    HS_CUDA(cudaLaunchCooperativeKernel(pcg_kernel(h, h->coop_grid < a.nruns), dim3(h->coop_grid), dim3(ST), args, pcg_smem(h->part.CX), h->s));
+    return HS_OK;
+}
+// a step's iteration count as k_step_end stores it: -1 where the cooperative
+// solve gave up waiting for a CTA
+hs_status check_iters(const int* it, int n) {
+    for (int i = 0; i < n; ++i)
+        if (it[i] < 0) { set_error("the PCG kernel gave up waiting for its other blocks"); return HS_ERR_CUDA; }
+    return HS_OK;
+}
+
 // build a graph: [rhs] + x0 matvec + prologue, then while(!done){ (K1; K2) x kLoopUnroll }.
 // Four iterations per pass of the while body spread the node's relaunch over
 // them (N=128: 70.6 -> 67.8 us per CG iteration); a solve that ends mid-pass
 // launches at most three iterations' kernels that return at once.
 constexpr int kLoopUnroll = 4;
 hs_status build_graph(hs_solver* h, int which) {
-    if (h->gexec[which] || !graphs_enabled()) return HS_OK;
+    if (h->gexec[which] || h->coop_grid || !graphs_enabled()) return HS_OK;
     const bool with_rhs = which == 0;
     cudaGraph_t g;
     HS_CUDA(cudaGraphCreate(&g, 0));
@@ -366,7 +451,7 @@ hs_status arm_step(hs_solver* h, const hs_fi_spec* fi, int step, bool allow_G) {
             c.vec = fi->level; c.iter = fi->iter; c.idx = (long long)(fi->target % h->Nn); c.bit = fi->bit;
         }
     }
-    k_step_begin<<<1, 1, 0, h->s>>>(h->st.p, c, h->T.p);
+    k_step_begin<<<1, 1, 0, h->s>>>(h->st.p, c, h->T.p, h->ticket.p + 64);
     HS_CUDA(cudaGetLastError());
     return HS_OK;
 }
@@ -497,15 +582,21 @@ hs_status hs_create(const hs_options* opt, const double* k_host, const double* r
     int dev = 0;
     HS_CUDA(cudaGetDevice(&dev));
     HS_CUDA(cudaDeviceGetAttribute(&h->n_sm, cudaDevAttrMultiProcessorCount, dev));
+    { hs_status cs = set_coop_grid(h.get(), dev); if (cs != HS_OK) return cs; }
     const size_t Nn = (size_t)h->Nn, Ne = (size_t)h->Ne;
     HS_CUDA(h->rhoc.alloc(Ne)); HS_CUDA(h->kc.alloc(Ne)); HS_CUDA(h->gtab.alloc(256)); HS_CUDA(h->coef.alloc(Ne));
     HS_CUDA(h->diag.alloc(Nn)); HS_CUDA(h->F.alloc(Nn));
     HS_CUDA(h->T.alloc(Nn)); HS_CUDA(h->b.alloc(Nn)); HS_CUDA(h->r.alloc(Nn)); HS_CUDA(h->z.alloc(Nn));
     HS_CUDA(h->p0.alloc(Nn)); HS_CUDA(h->p1.alloc(Nn)); HS_CUDA(h->Ap.alloc(Nn));
-    HS_CUDA(h->partials.alloc((size_t)MAXQ * std::max(h->part.nblk, h->part.nflat) + 4096));
-    HS_CUDA(h->upart.alloc((size_t)3 * h->part.nflat + 256));
-    HS_CUDA(h->ticket.alloc(1)); HS_CUDA(h->st.alloc(1)); HS_CUDA(h->red.alloc(8)); HS_CUDA(h->sp.alloc(2));
-    HS_CUDA(cudaMemsetAsync(h->ticket.p, 0, sizeof(unsigned), h->s));
+    HS_CUDA(h->partials.alloc((size_t)MAXQ * std::max(3 * h->part.nblk, h->part.nflat) + 4096));
+    // run sums, and the cooperative solve's exchange words (zero: no launch's tag)
+    const size_t n_upart = ((size_t)3 * h->part.nflat + 256 + 1) & ~(size_t)1;
+    const size_t n_words = h->coop_grid ? (size_t)2 * h->part.nblk + (size_t)6 * h->part.nflat : 0;
+    HS_CUDA(h->upart.alloc(n_upart + 2 * n_words));
+    h->xwords = reinterpret_cast<XWord*>(h->upart.p + n_upart);
+    HS_CUDA(cudaMemsetAsync(h->xwords, 0, n_words * sizeof(XWord), h->s));
+    HS_CUDA(h->ticket.alloc(128)); HS_CUDA(h->st.alloc(1)); HS_CUDA(h->red.alloc(8)); HS_CUDA(h->sp.alloc(2));
+    HS_CUDA(cudaMemsetAsync(h->ticket.p, 0, 128 * sizeof(unsigned), h->s));
     HS_CUDA(cudaMemsetAsync(h->st.p, 0, sizeof(DevState), h->s));
     for (DevBuf<double>* v : {&h->T, &h->b, &h->r, &h->z, &h->p0, &h->p1, &h->Ap})
         HS_CUDA(cudaMemsetAsync(v->p, 0, Nn * sizeof(double), h->s));
@@ -616,7 +707,7 @@ hs_status hs_apply(hs_solver* s, const double* x, double* y, double dt_eff, int 
         return HS_OK;
     }
     const bool d1 = s->opt.detect != 0;
-    k_step_begin<<<1, 1, 0, s->s>>>(s->st.p, c, s->T.p);
+    k_step_begin<<<1, 1, 0, s->s>>>(s->st.p, c, s->T.p, s->ticket.p + 64);
     // dt_eff == 0 is the mass matrix: checksum against w_M (build_rhs), else w_A
     if (dt_eff == 0.0)
         apply_projected(s, ROLE_RHS, x, y, dt_eff, d1, s->wM.p, nullptr, 0.0);
@@ -643,7 +734,7 @@ hs_status hs_build_rhs(hs_solver* s, const double* T, double* b) {
     if (!s || !T || !b) return HS_ERR_ARG;
     const bool src = !s->opt.verify && !s->opt.no_source && s->has_F;
     const bool d1 = s->opt.detect != 0;
-    k_step_begin<<<1, 1, 0, s->s>>>(s->st.p, StepCtl{}, s->T.p);
+    k_step_begin<<<1, 1, 0, s->s>>>(s->st.p, StepCtl{}, s->T.p, s->ticket.p + 64);
     apply_projected(s, ROLE_RHS, T, b, 0.0, d1, s->wM.p, src ? s->F.p : nullptr, s->opt.dt);
     HS_CUDA(cudaGetLastError());
     HS_CUDA(cudaStreamSynchronize(s->s));
@@ -690,7 +781,10 @@ hs_status enqueue_step(hs_solver* h, const hs_fi_spec* fi, int step, int reproje
     hs_status st = arm_step(h, fi, step, true);
     if (st != HS_OK) return st;
     if (e0) HS_CUDA(cudaEventRecord(e0, h->s));
-    if (graphs_enabled()) {
+    if (h->coop_grid) {
+        st = launch_pcg(h, true);
+        if (st != HS_OK) return st;
+    } else if (graphs_enabled()) {
         HS_CUDA(cudaGraphLaunch(h->gexec[0], h->s));
     } else {
         st = pcg_direct(h, true);
@@ -730,7 +824,10 @@ hs_status hs_pcg(hs_solver* s, const double* b, double* x, int max_iter, double 
     if (s->pending_set) { fi = s->pending; fi.step = 0; pf = &fi; s->pending_set = false; }
     st = arm_step(s, pf, 0, false);
     if (st != HS_OK) return st;
-    if (graphs_enabled()) {
+    if (s->coop_grid) {
+        st = launch_pcg(s, false);
+        if (st != HS_OK) return st;
+    } else if (graphs_enabled()) {
         HS_CUDA(cudaGraphLaunch(s->gexec[1], s->s));
     } else {
         st = pcg_direct(s, false);
@@ -742,6 +839,7 @@ hs_status hs_pcg(hs_solver* s, const double* b, double* x, int max_iter, double 
     DevState hsx{};
     HS_CUDA(cudaMemcpyAsync(&hsx, s->st.p, sizeof(hsx), cudaMemcpyDeviceToHost, s->s));
     HS_CUDA(cudaStreamSynchronize(s->s));
+    if (hsx.stuck) { const int bad = -1; return check_iters(&bad, 1); }
     if (iters) *iters = hsx.result;
     return sync_state_config(s, s->opt.max_iter, s->opt.rtol);
 }
@@ -857,6 +955,8 @@ hs_status run_case_impl(hs_solver* h, int n_steps, int snap_every, const hs_fi_s
     std::vector<double> rec((size_t)std::max(n_steps, 1) * 8);
     HS_CUDA(cudaMemcpy(it.data(), d_it.p, n_steps * sizeof(int), cudaMemcpyDeviceToHost));
     HS_CUDA(cudaMemcpy(rec.data(), d_rec.p, (size_t)n_steps * 8 * 8, cudaMemcpyDeviceToHost));
+    st = check_iters(it.data() + s0, n_steps - s0);
+    if (st != HS_OK) return st;
     int nf = 0;
     si = 0;
     if (keep_reference) { h->ref_tmin.assign(n_steps, 0.0); h->ref_tmax.assign(n_steps, 0.0); }
@@ -921,6 +1021,8 @@ hs_status hs_verify(hs_solver* h, int n_steps, double* rel_err, long long* total
     HS_CUDA(cudaEventElapsedTime(&fms, e0, e1));
     std::vector<int> it(std::max(n_steps, 1));
     HS_CUDA(cudaMemcpy(it.data(), d_it.p, n_steps * sizeof(int), cudaMemcpyDeviceToHost));
+    st = check_iters(it.data(), n_steps);
+    if (st != HS_OK) return st;
     long long tot = 0;
     for (int i = 0; i < n_steps; ++i) tot += it[i];
     // error against exp(-3 pi^2 alpha t) sin sin sin (het.cu:1314-1320)
@@ -964,6 +1066,8 @@ hs_status hs_solve_host(hs_solver* h, const double* T0_host, double* T_host, int
     HS_CUDA(cudaEventElapsedTime(&fms, e0, e1));
     std::vector<int> it(std::max(n_steps, 1));
     HS_CUDA(cudaMemcpy(it.data(), d_it.p, n_steps * sizeof(int), cudaMemcpyDeviceToHost));
+    st = check_iters(it.data(), n_steps);
+    if (st != HS_OK) return st;
     long long tot = 0;
     for (int i = 0; i < n_steps; ++i) tot += it[i];
     if (total_iters) *total_iters = tot;
@@ -1027,6 +1131,8 @@ hs_status hs_diag_cg(hs_solver* h, int max_iter, double tol, double* rel0, doubl
     HS_CUDA(cudaStreamSynchronize(h->s));
     int it = 0;
     HS_CUDA(cudaMemcpy(&it, d_it.p, sizeof(int), cudaMemcpyDeviceToHost));
+    st = check_iters(&it, 1);
+    if (st != HS_OK) return st;
     HS_CUDA(cudaMemcpy(&hsx, h->st.p, sizeof(hsx), cudaMemcpyDeviceToHost));
     const int n = std::min(it, cap);
     if (rel && n) HS_CUDA(cudaMemcpy(rel, lg.p, n * 8, cudaMemcpyDeviceToHost));
@@ -1086,6 +1192,8 @@ hs_status hs_advance(hs_solver* h, int n_steps, int from_ic, long long* total_it
     HS_CUDA(cudaEventElapsedTime(&fms, e0, e1));
     std::vector<int> it(std::max(n_steps, 1));
     HS_CUDA(cudaMemcpy(it.data(), d_it.p, n_steps * sizeof(int), cudaMemcpyDeviceToHost));
+    st = check_iters(it.data(), n_steps);
+    if (st != HS_OK) return st;
     long long tot = 0;
     for (int i = 0; i < n_steps; ++i) tot += it[i];
     if (total_iters) *total_iters = tot;
