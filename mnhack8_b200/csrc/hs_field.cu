@@ -41,17 +41,125 @@ __global__ void k_field_noise(long long ne, unsigned long long seed, double* g) 
     }
 }
 
-// one periodic 1-D Gaussian pass along axis (0: x, 1: y, 2: z) of an n^3
-// grid: out[i] = sum_t w(t) in[i + t e_axis mod n], t = -R..R, w(t) =
-// exp(-t^2 / (2 s^2)) (s in cells), weights built once per block
+// The weights of a pass: w(t) = exp(-t^2 / (2 s^2)), t = -R..R (s in cells)
 constexpr int kFieldMaxTaps = 4096;
-__global__ void k_field_conv(int n, int axis, int R, double s, const double* in, double* out) {
-    __shared__ double w[kFieldMaxTaps];
-    const int taps = 2 * R + 1;
-    for (int t = threadIdx.x; t < taps; t += blockDim.x) {
+__device__ __forceinline__ void field_weights(int R, double s, double* w) {
+    for (int t = threadIdx.x; t < 2 * R + 1; t += blockDim.x) {
         const double d = (double)(t - R);
         w[t] = exp(-d * d / (2.0 * s * s));
     }
+}
+
+// one periodic 1-D Gaussian pass along axis (0: x, 1: y, 2: z) of an n^3
+// grid: out[i] = sum_t w(t) in[i + t e_axis mod n], t = -R..R in order.
+// A block takes FL lines and up to FO outputs of each: the inputs with their
+// halo (wrapped) go to shared memory once, a lane works on one line and
+// carries FU consecutive outputs with a sliding window, so a tap costs one
+// shared load, one broadcast of its weight and FU multiply-adds.  Bound: the
+// shared-memory pipe and FP64 issue about equally (N=128, 49 taps: 103 M
+// multiply-adds a pass, 6 us of the FP64 pipe; 20 us measured, 38 us with the
+// window loaded one row at a time).  With one thread per output, a global load
+// and a wrap test per tap, the generator took 310 us of device time at N=128
+// and 1300 at N=160 with 97 taps; now 130 and 290.
+constexpr int FL = 32, FU = 8, FO = 8 * FU;      // one chunk of FU outputs per warp, 8 warps
+constexpr int kFieldPitch = FL + 1;      // z pass: lanes load along the line, so an odd pitch
+// outputs of a block along a line: the line in equal parts of at most FO, whole chunks
+__host__ __device__ inline int field_outs(int n) {
+    const int parts = (n + FO - 1) / FO;
+    return ((n + parts - 1) / parts + FU - 1) / FU * FU;
+}
+inline size_t field_conv_smem(int n, int R) {
+    return ((size_t)(field_outs(n) + 2 * R) * kFieldPitch + 2 * R + 1) * sizeof(double);
+}
+__global__ void __launch_bounds__(256) k_field_conv(int n, int axis, int R, double s, const double* in, double* out) {
+    extern __shared__ __align__(16) double sm[];
+    const int outs = field_outs(n);
+    const int span = outs + 2 * R, taps = 2 * R + 1;
+    double* S = sm;                                           // [span][kFieldPitch]
+    double* w = sm + (size_t)span * kFieldPitch;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const long long nn = (long long)n * n;
+    const long long line0 = (long long)blockIdx.x * FL;
+    const int o0 = blockIdx.y * outs;                         // first output
+    const long long stride = axis == 0 ? nn : axis == 1 ? (long long)n : 1;
+    // first element of line l (lines in the order of the other two axes)
+    auto base = [&](long long l) { return axis == 0 ? l : axis == 1 ? (l / n) * nn + l % n : l * n; };
+    field_weights(R, s, w);
+    // rows of the window: z takes a warp per line with the lanes along it, the
+    // other axes a warp per row with the lanes across the lines; BL loads in flight
+    constexpr int BL = 7;
+    const int step = axis == 2 ? 32 : 8, inc = step % n;
+    for (int q = axis == 2 ? warp : lane; q < FL; q += axis == 2 ? 8 : FL) {
+        const long long ln = line0 + q;
+        const double* src = in + base(ln < nn ? ln : 0);
+        int i = axis == 2 ? lane : warp;
+        int c = (((o0 - R + i) % n) + n) % n;
+        while (i < span) {
+            double v[BL];
+#pragma unroll
+            for (int b = 0; b < BL; ++b) {
+                v[b] = (i + b * step < span) ? __ldg(src + (long long)c * stride) : 0.0;
+                c += inc;
+                if (c >= n) c -= n;
+            }
+#pragma unroll
+            for (int b = 0; b < BL; ++b, i += step)
+                if (i < span) S[i * kFieldPitch + q] = v[b];
+        }
+    }
+    __syncthreads();
+    const int u0 = warp * FU;
+    const long long l = line0 + lane;
+    double acc[FU], win[FU];
+    if (u0 < outs) {
+        const double* L = S + (size_t)u0 * kFieldPitch + lane;
+#pragma unroll
+        for (int u = 0; u < FU; ++u) { acc[u] = 0.0; win[u] = L[u * kFieldPitch]; }
+        // taps (odd) = whole groups of FU and a rest; the last tap needs no new input
+        int t0 = 0;
+        for (; t0 + FU < taps; t0 += FU) {
+#pragma unroll
+            for (int tt = 0; tt < FU; ++tt) {
+                const double wt = w[t0 + tt], nx = L[(t0 + tt + FU) * kFieldPitch];
+#pragma unroll
+                for (int u = 0; u < FU; ++u) acc[u] = __fma_rn(wt, win[(u + tt) % FU], acc[u]);
+                win[tt] = nx;
+            }
+        }
+#pragma unroll
+        for (int tt = 0; tt < FU; ++tt) {
+            if (t0 + tt < taps) {
+                const double wt = w[t0 + tt];
+#pragma unroll
+                for (int u = 0; u < FU; ++u) acc[u] = __fma_rn(wt, win[(u + tt) % FU], acc[u]);
+                if (t0 + tt + 1 < taps) win[tt] = L[(t0 + tt + FU) * kFieldPitch];
+            }
+        }
+        if (axis != 2 && l < nn) {
+#pragma unroll
+            for (int u = 0; u < FU; ++u)
+                if (o0 + u0 + u < n) out[base(l) + (long long)(o0 + u0 + u) * stride] = acc[u];
+        }
+    }
+    if (axis != 2) return;
+    // z: turned in shared memory, so that the stores run along the lines
+    __syncthreads();
+    if (u0 < outs) {
+#pragma unroll
+        for (int u = 0; u < FU; ++u) S[(u0 + u) * kFieldPitch + lane] = acc[u];
+    }
+    __syncthreads();
+    for (int q = warp; q < FL; q += 8) {
+        if (line0 + q >= nn) break;
+        for (int i = lane; i < outs && o0 + i < n; i += 32) out[base(line0 + q) + o0 + i] = S[i * kFieldPitch + q];
+    }
+}
+
+// The same pass for kernels too wide for the window to fit in shared memory.
+__global__ void k_field_conv_wide(int n, int axis, int R, double s, const double* in, double* out) {
+    __shared__ double w[kFieldMaxTaps];
+    const int taps = 2 * R + 1;
+    field_weights(R, s, w);
     __syncthreads();
     const long long nn = (long long)n * n, ne = nn * n;
     const long long stride = axis == 0 ? nn : axis == 1 ? (long long)n : 1;
@@ -95,11 +203,14 @@ __global__ void __launch_bounds__(RT) k_field_moment_final(long long ne, int pas
     if (pass == 0) stats[0] = __ddiv_rn(v[0], (double)ne);
     else stats[1] = __dsqrt_rn(__ddiv_rn(v[0], (double)ne));
 }
-// k = exp(mu + sigma (g - mean) / std), rho*c = rhoc (g is read from rh)
-__global__ void k_field_finish(long long ne, double mu, double sigma, double rhoc, const double* stats, double* k,
-                               double* rh) {
+// k = exp(mu + sigma (g - mean) / std), rho*c = rhoc (g is read from rh) for
+// elements e0 .. e1-1.  stats may be elements of k: outside the launch's range,
+// or in that of a launch of one block.
+__global__ void k_field_finish(long long e0, long long e1, double mu, double sigma, double rhoc, const double* stats,
+                               double* k, double* rh) {
     const double mean = stats[0], sd = stats[1];
-    for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < ne; e += (long long)gridDim.x * blockDim.x) {
+    __syncthreads();
+    for (long long e = e0 + (long long)blockIdx.x * blockDim.x + threadIdx.x; e < e1; e += (long long)gridDim.x * blockDim.x) {
         const double g = __ddiv_rn(dsub(rh[e], mean), sd);
         k[e] = exp(dfma(sigma, g, mu));
         rh[e] = rhoc;
@@ -123,7 +234,9 @@ inline void field_taps(int n, double L, int* R, double* s) {
 
 // Enqueue a lognormal field on stream st into k and rh (N^3 doubles each; rh
 // is also the working buffer).  partials: ceil(N^3 / (RT*KF)) doubles;
-// stats: 2 doubles.
+// stats: 2 doubles; both null: k itself holds them until its values are written
+// (N >= 2), so that no scratch memory is needed (allocating and freeing it took
+// 600 us of a call).
 inline cudaError_t enqueue_field_lognormal(const FieldSpecDev& f, double* k, double* rh, double* partials,
                                            double* stats, cudaStream_t st) {
     const int n = f.N;
@@ -132,16 +245,32 @@ inline cudaError_t enqueue_field_lognormal(const FieldSpecDev& f, double* k, dou
     int R = 1;
     double s = 1.0;
     field_taps(n, f.L, &R, &s);
+    const long long tail = stats ? 0 : 2;
+    if (!stats) { partials = k; stats = k + ne - 2; }       // k is free after the last pass
     const int g = (int)std::min<long long>((ne + RT - 1) / RT, 148 * 32);
     k_field_noise<<<g, RT, 0, st>>>(ne, f.seed, k);
-    k_field_conv<<<g, RT, 0, st>>>(n, 2, R, s, k, rh);    // z
-    k_field_conv<<<g, RT, 0, st>>>(n, 1, R, s, rh, k);    // y
-    k_field_conv<<<g, RT, 0, st>>>(n, 0, R, s, k, rh);    // x
+    // the window fits in shared memory up to a reach of 390 cells (a correlation of 130 cells)
+    const size_t smem = field_conv_smem(n, R);
+    constexpr size_t most = 220 * 1024;
+    const bool fits = smem <= most;
+    if (fits) {
+        const cudaError_t e = cudaFuncSetAttribute(k_field_conv, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+        if (e != cudaSuccess) return e;
+    }
+    auto conv = [&](int axis, const double* in, double* out) {
+        const dim3 grid((unsigned)(((long long)n * n + FL - 1) / FL), (unsigned)((n + field_outs(n) - 1) / field_outs(n)));
+        if (fits) k_field_conv<<<grid, 256, smem, st>>>(n, axis, R, s, in, out);
+        else k_field_conv_wide<<<g, RT, 0, st>>>(n, axis, R, s, in, out);
+    };
+    conv(2, k, rh);    // z
+    conv(1, rh, k);    // y
+    conv(0, k, rh);    // x
     for (int pass = 0; pass < 2; ++pass) {
         k_field_moment<<<(int)nblk, RT, 0, st>>>(ne, pass, rh, stats, partials, nblk);
         k_field_moment_final<<<1, RT, 0, st>>>(ne, pass, partials, nblk, stats);
     }
-    k_field_finish<<<g, RT, 0, st>>>(ne, f.mu, f.sigma, f.rhoc, stats, k, rh);
+    k_field_finish<<<g, RT, 0, st>>>(0, ne - tail, f.mu, f.sigma, f.rhoc, stats, k, rh);
+    if (tail) k_field_finish<<<1, 32, 0, st>>>(ne - tail, ne, f.mu, f.sigma, f.rhoc, stats, k, rh);
     return cudaGetLastError();
 }
 
@@ -154,15 +283,14 @@ extern "C" hs_status hs_field_lognormal(int N, double mu, double sigma, double L
         set_error("hs_field_lognormal: bad arguments");
         return HS_ERR_ARG;
     }
-    const long long ne = (long long)N * N * N;
-    const long long nblk = (ne + (long long)RT * KF - 1) / ((long long)RT * KF);
     double* scratch = nullptr;
-    cudaError_t e = cudaMalloc(&scratch, (size_t)(nblk + 2) * sizeof(double));
-    if (e != cudaSuccess) { set_error(std::string("hs_field_lognormal: ") + cudaGetErrorString(e)); return HS_ERR_CUDA; }
+    cudaError_t e = cudaSuccess;
+    if (N == 1) e = cudaMalloc(&scratch, 3 * sizeof(double));      // one element holds no scratch
     FieldSpecDev f{N, mu, sigma, L, rhoc, seed};
-    e = enqueue_field_lognormal(f, k_dev, rhoc_dev, scratch + 2, scratch, 0);
+    if (e == cudaSuccess)
+        e = enqueue_field_lognormal(f, k_dev, rhoc_dev, scratch ? scratch + 2 : nullptr, scratch, 0);
     if (e == cudaSuccess) e = cudaStreamSynchronize(0);
-    cudaFree(scratch);
+    if (scratch) cudaFree(scratch);
     if (e != cudaSuccess) { set_error(std::string("hs_field_lognormal: ") + cudaGetErrorString(e)); return HS_ERR_CUDA; }
     return HS_OK;
 }
