@@ -304,6 +304,8 @@ struct ApplyArgs {
     double* pbuf1;
     double* y;              // output
     const double2* coef;    // per element (rho*c, k)
+    const double* kc;       // uniform rho*c: per element k
+    double rc;              // and its value
     const double* w;        // ABFT weight (w_M or w_A) or null
     const double* F;        // ROLE_RHS source (null: none)
     double dtF;
@@ -317,45 +319,72 @@ struct ApplyArgs {
 // ---- colored operator: slab tiles ------------------------------------------------
 // One CTA of ST threads streams a tile's node planes in increasing x.  Per
 // element layer ix (between planes ix and ix+1):
-//   1. plane ix+1 is formed (p = z + beta p_{k-1} in the PCG loop) from
-//      registers loaded one layer ahead, kept in registers and published to
-//      shared memory;
-//   2. the element whose lower corner is a position (own column) gathers its
-//      six other corners from the two published planes, applies the element
-//      operator, folds its own-column outputs (q = 0 into the plane-ix node,
-//      q = 4 into the plane-(ix+1) node) into per-position accumulators and
-//      hands the other six to the three neighbouring positions;
-//   3. each tile node of plane ix adds the three handed-in contributions
-//      (q = 3, 2, 1), which completes its canonical node sum, and is
-//      projected, checked and stored; the plane-(ix+1) accumulators take
-//      q = 7, 6, 5.
-// Per node and layer that is one shared store of p, six shared loads for the
-// gather and three 16-byte stores and loads for the hand-over.
+//   1. the element whose lower corner is a position gathers its corners from
+//      the two published planes, applies the element operator, folds its
+//      own-column outputs (q = 0 into the plane-ix node, q = 4 into the
+//      plane-(ix+1) node) into per-position accumulators and hands the other
+//      six to the three neighbouring positions;
+//   2. plane ix+2 is formed (p = z + beta p_{k-1} in the PCG loop) from
+//      registers loaded one layer ahead, published in the third plane buffer,
+//      and its tile nodes are stored and added to w.p and p.p;
+//   3. after the layer's one CTA barrier each tile node of plane ix adds the
+//      three handed-in contributions (q = 3, 2, 1), which completes its
+//      canonical node sum, and is projected, checked and stored; the
+//      plane-(ix+1) accumulators take q = 7, 6, 5.
+// The hand-over buffers are written again in the next layer's step 1: a warp
+// announces on an mbarrier that it has read them and waits for the others only
+// before its first store there, behind its gathers and element arithmetic, so
+// that wait costs nothing and warps may be in different steps.
+//
+// What bounds it: instruction issue and latency with 16 warps per SM (128
+// registers a thread), and the shared-memory pipe (74 % busy at N=256), not the
+// DRAM traffic, which is the algorithmic minimum.  Measured (B200, PCG-loop role with
+// checksum, L2 scrubbed, uniform rho*c, before -> after): N=97 26.7 -> 24.7 us,
+// N=128 42.5 -> 38.3, N=256 245 -> 210 to 218; a plain apply at N=256 241 -> 182.
+// Of that, one barrier per layer in place of two and the p-only work moved from
+// step 3 into step 2 (its checksum weight no longer waited for: long-scoreboard
+// stalls 2.35 -> 0.60 per issue) gave 245 -> 225, the uniform rho*c form and the
+// checksum as a template argument (177 -> 160 instructions per position) the
+// rest.  Tried on top and not faster: forming each plane's z and y butterflies
+// once (8 FP64 operations and 4 shared loads fewer, but 24 registers more: spills
+// or moves), the own column's p in registers, clamped unconditional loads,
+// branch-free node sums.
 struct __align__(16) SlabSmem {
-    double P[2][SPOS];      // formed planes, plane px in P[px & 1]
+    double P[3][SPOS];      // formed planes, three in turn
     double2 Y1[SPOS];       // from the element at position j-1:      (q1, q5)
     double2 Y2[SPOS];       // from the element at position j-Cw:     (q2, q6)
     double2 Y3[SPOS];       // from the element at position j-Cw-1:   (q3, q7)
     double sh[MAXQ][8];
+    unsigned long long free_bar;
 };
-constexpr size_t kSlabSmem = sizeof(SlabSmem);
-
-// A load of a vector: read-only for the kernel's whole life (the non-coherent
-// path), or, with COH, written by other CTAs of the same launch before a grid
-// barrier (through the L2, past a possibly stale L1 line).
-template <bool COH, typename V>
-__device__ __forceinline__ V ld_vec(const V* p) {
-    if constexpr (COH) return __ldcg(p);
-    else return __ldg(p);
+__device__ __forceinline__ void mbar_init(unsigned b, unsigned n) {
+    asm volatile("mbarrier.init.shared.b64 [%0], %1;" ::"r"(b), "r"(n) : "memory");
 }
+__device__ __forceinline__ void mbar_inval(unsigned b) { asm volatile("mbarrier.inval.shared.b64 [%0];" ::"r"(b) : "memory"); }
+__device__ __forceinline__ void mbar_arrive(unsigned b) {
+    asm volatile("{\n\t.reg .b64 t;\n\tmbarrier.arrive.shared.b64 t, [%0];\n\t}" ::"r"(b) : "memory");
+}
+// Waits for the phase of parity `phase`, in which every warp of the CTA arrives;
+// false after about a second
+__device__ __forceinline__ bool mbar_wait(unsigned b, unsigned phase) {
+    unsigned ok = 0, left = 1u << 22;
+    do {
+        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                     : "=r"(ok) : "r"(b), "r"(phase) : "memory");
+    } while (!ok && --left);
+    return ok != 0u;
+}
+constexpr size_t kSlabSmem = sizeof(SlabSmem);
 
 // MODE 0: input x as given; 1: PCG loop, p = z; 2: PCG loop, p = z + beta p_{k-1}.
 // FI false: no fault is armed for this launch (the per-node fault tests compile out).
-// COH: the input vectors are written inside this launch (ld_vec).
-template <int FORM, int MODE, bool FI = true, bool COH = false>
+// RC: rho*c is one value (a.rc), so only k is read per element and rho*c's
+// products with the eigen-constants are formed once (N=128 40.9 -> 39.5 us; the
+// same operations on the same values).  D1: the checksum sums are taken.
+template <int FORM, int MODE, bool FI, bool RC, bool D1>
 __device__ __forceinline__ void slab_march(const ApplyArgs& a, SlabSmem& S, const SlabTile& T, const SlabPos& G,
                                            const double* src_a, const double* src_b, double beta, double* pout,
-                                           bool loop, bool d1, bool rhs, int fi_p, int fi_ap, int fi_r, int fi_bit,
+                                           bool loop, bool rhs, int fi_p, int fi_ap, int fi_r, int fi_bit,
                                            long long fi_idx, long long fi_elem, double (&part)[MAXQ]) {
     constexpr bool TWO = MODE == 2;
     if (!FI) { fi_p = 0; fi_ap = 0; fi_r = 0; }
@@ -367,24 +396,38 @@ __device__ __forceinline__ void slab_march(const ApplyArgs& a, SlabSmem& S, cons
     const unsigned fl = G.fl;
     const int xa = T.xa, xb = T.xb;
 
-    double pA[SK], pB[SK], aA[SK], aB[SK], ra[SK], rb[SK], cr[SK], ck[SK], wv[SK], fv[SK];
-    auto ld_raw = [&](int px) {
-        const bool pv = px >= 0 && px <= N;
+    double ra[SK], rb[SK], cr[SK], ck[SK], wv[SK], fv[SK];
+    // raw inputs of plane px (z, p_{k-1}; the checksum weight and the source of
+    // its tile nodes), loaded a layer before they are used
+    auto ld_raw = [&](int px, double (&ra)[SK], double (&rb)[SK], double (&wv)[SK]) {
+        const bool pv = px >= 0 && px <= N, pt = px >= xa && px <= xb;
         const unsigned base = (unsigned)px * plane;
 #pragma unroll
         for (int k = 0; k < SK; ++k) {
-            const bool v = pv && sp_valid(fl, k);
+            const bool v = pv && sp_valid(fl, k), o = pt && sp_out(fl, k);
             const unsigned n = base + (unsigned)G.noff[k];
-            ra[k] = v ? ld_vec<COH>(src_a + n) : 0.0;
-            if (TWO) rb[k] = v ? ld_vec<COH>(src_b + n) : 0.0;
+            ra[k] = v ? __ldg(src_a + n) : 0.0;
+            if (TWO) rb[k] = v ? __ldg(src_b + n) : 0.0;
+            wv[k] = (o && D1) ? __ldg(a.w + n) : 0.0;
         }
     };
-    auto form = [&](int px, double (&p)[SK]) {
+    // plane px of p (or x): formed, published, and for the tile's own nodes
+    // stored and added to w.p and p.p
+    auto form = [&](int px, double* P, const double (&ra)[SK], const double (&rb)[SK], const double (&wv)[SK]) {
+        const bool pt = px >= xa && px <= xb;
+        const unsigned base = (unsigned)px * plane;
 #pragma unroll
         for (int k = 0; k < SK; ++k) {
             double v = TWO ? dfma(beta, rb[k], ra[k]) : ra[k];
             if (fi_p && sp_valid(fl, k) && (long long)px * plane + G.noff[k] == fi_idx) v = flipbit(v, fi_bit);
-            p[k] = v;
+            P[tid + k * ST] = v;
+            if (pt && sp_out(fl, k)) {
+                if (D1) {
+                    part[2] = dfma(wv[k], v, part[2]);
+                    part[3] = dfma(v, v, part[3]);
+                }
+                if (TWO || MODE == 1) pout[base + (unsigned)G.noff[k]] = v;
+            }
         }
     };
     auto ld_coef = [&](int ex) {
@@ -393,34 +436,28 @@ __device__ __forceinline__ void slab_march(const ApplyArgs& a, SlabSmem& S, cons
 #pragma unroll
         for (int k = 0; k < SK; ++k) {
             const bool v = ev && sp_elem(fl, k);
-            const double2 c = v ? __ldg(a.coef + (base + (unsigned)G.eoff[k])) : make_double2(0.0, 0.0);
-            cr[k] = c.x; ck[k] = c.y;
+            if constexpr (RC) {
+                ck[k] = v ? __ldg(a.kc + (base + (unsigned)G.eoff[k])) : 0.0;
+            } else {
+                const double2 c = v ? __ldg(a.coef + (base + (unsigned)G.eoff[k])) : make_double2(0.0, 0.0);
+                cr[k] = c.x; ck[k] = c.y;
+            }
         }
     };
-    auto ld_w = [&](int px) {
+    auto ld_f = [&](int px) {
         const bool pv = px >= xa && px <= xb;
-        const unsigned base = (unsigned)px * plane;
 #pragma unroll
-        for (int k = 0; k < SK; ++k) {
-            const bool v = pv && sp_out(fl, k);
-            const unsigned n = base + (unsigned)G.noff[k];
-            wv[k] = (v && d1) ? __ldg(a.w + n) : 0.0;
-            if (MODE == 0) fv[k] = (v && rhs) ? __ldg(a.F + n) : 0.0;
-        }
+        for (int k = 0; k < SK; ++k)
+            fv[k] = (rhs && pv && sp_out(fl, k)) ? __ldg(a.F + ((unsigned)px * plane + (unsigned)G.noff[k])) : 0.0;
     };
 
-    // One element layer ix (between planes ix and ix+1).  Plane px lives in
-    // P[(px - xa + 1) & 1] (cur for plane ix); pc / pn hold planes ix / ix+1
-    // of the own column, ac / an the node sums of planes ix / ix+1.
-    auto layer = [&](int ix, int cur, double (&pc)[SK], double (&pn)[SK], double (&ac)[SK], double (&an)[SK]) {
-        const int nxt = cur ^ 1;
-        // 1. plane ix+1
-        form(ix + 1, pn);
-#pragma unroll
-        for (int k = 0; k < SK; ++k) S.P[nxt][tid + k * ST] = pn[k];
-        ld_raw(ix + 2 <= xb + 1 ? ix + 2 : -2);
-        __syncthreads();
-        // 2. element layer ix
+    const int lane = tid & 31;
+    const unsigned free_bar = (unsigned)__cvta_generic_to_shared(&S.free_bar);
+    unsigned phase = 0;
+    // ac: node sums of plane ix from layer ix-1.  P0, P1, P2: shared planes ix, ix+1, ix+2.
+    double ac[SK], an[SK];
+    auto layer = [&](int ix, double* P0, double* P1, double* P2) {
+        // element layer ix
         if (ix >= 0 && ix < N) {
 #pragma unroll
             for (int k = 0; k < SK; ++k) {
@@ -430,28 +467,36 @@ __device__ __forceinline__ void slab_march(const ApplyArgs& a, SlabSmem& S, cons
                 const bool ev = sp_elem(fl, k);
                 const int j = tid + k * ST;
                 double v[8];
-                v[0] = pc[k];
-                v[1] = S.P[cur][j + 1];
-                v[2] = S.P[cur][j + Cw];
-                v[3] = S.P[cur][j + Cw + 1];
-                v[4] = pn[k];
-                v[5] = S.P[nxt][j + 1];
-                v[6] = S.P[nxt][j + Cw];
-                v[7] = S.P[nxt][j + Cw + 1];
-                elem_apply<FORM>(v, cr[k], ck[k], a.dt_eff, a.ec);
+                v[0] = P0[j];
+                v[1] = P0[j + 1];
+                v[2] = P0[j + Cw];
+                v[3] = P0[j + Cw + 1];
+                v[4] = P1[j];
+                v[5] = P1[j + 1];
+                v[6] = P1[j + Cw];
+                v[7] = P1[j + Cw + 1];
+                elem_apply<FORM>(v, RC ? a.rc : cr[k], ck[k], a.dt_eff, a.ec);
                 if (fi_r && (long long)ix * eplane + G.eoff[k] == fi_elem) v[0] = flipbit(v[0], fi_bit);
                 ac[k] = dadd(ac[k], v[0]);
                 an[k] = dadd(0.0, v[4]);
+                if (k == 0 && ix >= xa && !mbar_wait(free_bar, phase)) a.st->stuck = 1;   // the hand-over buffers are free again
                 if (ev) {
                     S.Y1[j + 1] = make_double2(v[1], v[5]);
                     S.Y2[j + Cw] = make_double2(v[2], v[6]);
                     S.Y3[j + Cw + 1] = make_double2(v[3], v[7]);
                 }
             }
+        } else {
+#pragma unroll
+            for (int k = 0; k < SK; ++k) an[k] = 0.0;
+            if (ix >= xa && !mbar_wait(free_bar, phase)) a.st->stuck = 1;
         }
+        if (ix >= xa) phase ^= 1u;
         ld_coef(ix + 1 <= xb ? ix + 1 : -1);
+        form(ix + 2, P2, ra, rb, wv);
+        ld_raw(ix + 3 <= xb + 1 ? ix + 3 : -2, ra, rb, wv);
         __syncthreads();
-        // 3. tile nodes of plane ix; node sums of plane ix+1
+        // tile nodes of plane ix; node sums of plane ix+1
         const unsigned base = (unsigned)ix * plane;
         const bool xbnd = ix == 0 || ix == N;
 #pragma unroll
@@ -466,48 +511,52 @@ __device__ __forceinline__ void slab_march(const ApplyArgs& a, SlabSmem& S, cons
                 const bool bnd = !yzin || xbnd;
                 double y = bnd ? 0.0 : dadd(dadd(dadd(ac[k], y3.x), y2.x), y1.x);
                 if (fi_ap && (long long)n == fi_idx) y = flipbit(y, fi_bit);
-                const double pv = pc[k];
-                if (loop) part[0] = dfma(pv, y, part[0]);
-                if (d1) {
-                    part[1] = bnd ? dfma(0.0, y, part[1]) : dadd(part[1], y);
-                    part[2] = dfma(wv[k], pv, part[2]);
-                    part[3] = dfma(pv, pv, part[3]);
-                }
+                if (loop) part[0] = dfma(P0[j], y, part[0]);
+                if (D1) part[1] = bnd ? dfma(0.0, y, part[1]) : dadd(part[1], y);
                 if (MODE == 0 && rhs) y = dfma(a.dtF, fv[k], y);
                 a.y[n] = y;
-                if (TWO || MODE == 1) pout[n] = pv;
             }
-            an[k] = yzin ? dadd(dadd(dadd(an[k], y3.y), y2.y), y1.y) : 0.0;
+            ac[k] = yzin ? dadd(dadd(dadd(an[k], y3.y), y2.y), y1.y) : 0.0;
         }
-        ld_w(ix + 1);
+        __syncwarp();
+        if (lane == 0) mbar_arrive(free_bar);
+        if (MODE == 0) ld_f(ix + 1);
     };
 
-    // plane xa-1, then the inputs of plane xa and the coefficients of layer xa-1
-    ld_raw(xa - 1);
-    form(xa - 1, pA);
+    if (tid == 0) mbar_init(free_bar, ST / 32);
+    double *P0 = S.P[0], *P1 = S.P[1], *P2 = S.P[2];
 #pragma unroll
-    for (int k = 0; k < SK; ++k) { S.P[0][tid + k * ST] = pA[k]; aA[k] = 0.0; aB[k] = 0.0; }
-    ld_raw(xa);
-    ld_coef(xa - 1);
-    for (int ix = xa - 1; ix <= xb; ++ix) {
-        layer(ix, (ix - xa + 1) & 1, pA, pB, aA, aB);
-#pragma unroll
-        for (int k = 0; k < SK; ++k) { pA[k] = pB[k]; aA[k] = aB[k]; }
+    for (int k = 0; k < SK; ++k) ac[k] = 0.0;
+    {
+        // the first two planes' loads together, then the third's
+        double ra0[SK], rb0[SK], wv0[SK];
+        ld_raw(xa - 1, ra0, rb0, wv0);
+        ld_raw(xa, ra, rb, wv);
+        ld_coef(xa - 1);
+        form(xa - 1, P0, ra0, rb0, wv0);
+        form(xa, P1, ra, rb, wv);
+        ld_raw(xa + 1, ra, rb, wv);
     }
+    __syncthreads();
+    for (int ix = xa - 1; ix <= xb; ++ix) {
+        layer(ix, P0, P1, P2);
+        double* t = P0; P0 = P1; P1 = P2; P2 = t;
+    }
+    __syncthreads();
+    if (tid == 0) mbar_inval(free_bar);
 }
 
 // Colored operator: tile blockIdx.x of the slab partition (every node of the
 // grid belongs to exactly one tile; boundary nodes are projected to zero).
 // LOOP: the PCG-loop role (p formed in the kernel); otherwise the roles that
 // apply the operator to a given vector.
-template <int FORM, bool LOOP>
+template <int FORM, bool LOOP, bool RC, bool D1>
 __global__ void __launch_bounds__(ST, FORM == FORM_WHT ? 2 : 1) k_apply_slab(ApplyArgs a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     SlabSmem& S = *reinterpret_cast<SlabSmem*>(smem_raw);
     DevState* st = a.st;
     int fi_p = 0, fi_ap = 0, fi_r = 0, fi_bit = 0;
     long long fi_idx = -1, fi_elem = -1;
-    const bool d1 = a.d1 != 0;
     double part[MAXQ] = {0.0, 0.0, 0.0, 0.0};
     const SlabTile T = slab_tile(a.part, blockIdx.x);
     const SlabPos G = slab_pos(a.part, T, threadIdx.x);
@@ -524,19 +573,19 @@ __global__ void __launch_bounds__(ST, FORM == FORM_WHT ? 2 : 1) k_apply_slab(App
             fi_p = (st->fi_vec == FI_P); fi_ap = (st->fi_vec == FI_AP);
         }
         if (!src_b)
-            slab_march<FORM, 1>(a, S, T, G, a.z, src_b, beta, pout, true, d1, false, fi_p, fi_ap, 0, fi_bit, fi_idx,
+            slab_march<FORM, 1, true, RC, D1>(a, S, T, G, a.z, src_b, beta, pout, true, false, fi_p, fi_ap, 0, fi_bit, fi_idx,
                                 -1, part);
         else if (fi_p || fi_ap)
-            slab_march<FORM, 2, true>(a, S, T, G, a.z, src_b, beta, pout, true, d1, false, fi_p, fi_ap, 0, fi_bit,
+            slab_march<FORM, 2, true, RC, D1>(a, S, T, G, a.z, src_b, beta, pout, true, false, fi_p, fi_ap, 0, fi_bit,
                                       fi_idx, -1, part);
         else
-            slab_march<FORM, 2, false>(a, S, T, G, a.z, src_b, beta, pout, true, d1, false, 0, 0, 0, 0, -1, -1, part);
+            slab_march<FORM, 2, false, RC, D1>(a, S, T, G, a.z, src_b, beta, pout, true, false, 0, 0, 0, 0, -1, -1, part);
     } else {
         if (a.role == ROLE_X0 && st->fi_armR) { fi_r = 1; fi_elem = st->fi_elem; fi_bit = st->fi_bit; }
         const bool rhs = (a.role == ROLE_RHS) && a.F != nullptr;
-        slab_march<FORM, 0>(a, S, T, G, a.x, nullptr, 0.0, nullptr, false, d1, rhs, 0, 0, fi_r, fi_bit, -1, fi_elem,
+        slab_march<FORM, 0, true, RC, D1>(a, S, T, G, a.x, nullptr, 0.0, nullptr, false, rhs, 0, 0, fi_r, fi_bit, -1, fi_elem,
                             part);
-        if (!d1) return;
+        if (!D1) return;
     }
     store_partials<MAXQ>(part, a.partials, a.part.nblk, S.sh);
 }
@@ -632,84 +681,62 @@ struct UpdStep {
     long long fi_idx;
 };
 
-// The update of U flat blocks at once (U > 1: of U different runs, so that
-// their loads are in flight together): each thread takes its KF consecutive
-// nodes of each block (KF / 2 aligned 128-bit loads and stores per vector), in
-// order, and carries on its run's sums in part (PRE: b.b, r.z, r.r; LOOP: r.r,
-// r.z).  A block index of nflat or more is no block.
-template <int U, bool COH>
-__device__ __forceinline__ void upd_blocks(const UpdateArgs& a, const UpdStep& s, const long long (&blk)[U],
-                                           double (&part)[U][3]) {
+// The update of one flat block: each thread takes its KF consecutive nodes
+// (KF / 2 aligned 128-bit loads and stores per vector), in order, and carries
+// on its run's sums in part (PRE: b.b, r.z, r.r; LOOP: r.r, r.z).
+__device__ __forceinline__ void upd_block(const UpdateArgs& a, const UpdStep& s, long long blk, double (&part)[3]) {
     static_assert(KF == 2, "one pair of nodes per thread and block");
-    const int tid = threadIdx.x;
-    long long m0[U];
-    int cnt[U];
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-        m0[u] = (blk[u] * RT + tid) * KF;
-        cnt[u] = (blk[u] >= a.nflat) ? 0 : (m0[u] + 1 < a.Nn) ? 2 : (m0[u] < a.Nn ? 1 : 0);
-    }
-    auto ld = [&](const double* base, double (&v)[U][KF]) {
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-            if (cnt[u] == 2) {
-                const double2 t = ld_vec<COH>(reinterpret_cast<const double2*>(base + m0[u]));
-                v[u][0] = t.x; v[u][1] = t.y;
-            } else { v[u][0] = cnt[u] ? ld_vec<COH>(base + m0[u]) : 0.0; v[u][1] = 0.0; }
-        }
+    const long long m0 = (blk * RT + threadIdx.x) * KF;
+    const int cnt = (m0 + 1 < a.Nn) ? 2 : (m0 < a.Nn ? 1 : 0);
+    auto ld = [&](const double* base, double (&v)[KF]) {
+        if (cnt == 2) {
+            const double2 t = __ldg(reinterpret_cast<const double2*>(base + m0));
+            v[0] = t.x; v[1] = t.y;
+        } else { v[0] = cnt ? __ldg(base + m0) : 0.0; v[1] = 0.0; }
     };
-    auto stv = [&](double* base, const double (&v)[U][KF]) {
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-            if (cnt[u] == 2) *reinterpret_cast<double2*>(base + m0[u]) = make_double2(v[u][0], v[u][1]);
-            else if (cnt[u] == 1) base[m0[u]] = v[u][0];
-        }
+    auto stv = [&](double* base, const double (&v)[KF]) {
+        if (cnt == 2) *reinterpret_cast<double2*>(base + m0) = make_double2(v[0], v[1]);
+        else if (cnt == 1) base[m0] = v[0];
     };
     if (s.pre) {
-        double bb[U][KF], qq[U][KF], dd[U][KF];
+        double bb[KF], qq[KF], dd[KF];
         ld(a.b, bb); ld(a.Ap, qq); ld(a.d, dd);
 #pragma unroll
-        for (int u = 0; u < U; ++u)
-#pragma unroll
-            for (int k = 0; k < KF; ++k) {
-                if (k >= cnt[u]) continue;
-                const double r_ = dfma(-1.0, qq[u][k], bb[u][k]);
-                const double z_ = __ddiv_rn(r_, dd[u][k]);
-                part[u][0] = dfma(bb[u][k], bb[u][k], part[u][0]);
-                part[u][1] = dfma(r_, z_, part[u][1]);
-                part[u][2] = dfma(r_, r_, part[u][2]);
-                qq[u][k] = r_; dd[u][k] = z_;
-            }
+        for (int k = 0; k < KF; ++k) {
+            if (k >= cnt) continue;
+            const double r_ = dfma(-1.0, qq[k], bb[k]);
+            const double z_ = __ddiv_rn(r_, dd[k]);
+            part[0] = dfma(bb[k], bb[k], part[0]);
+            part[1] = dfma(r_, z_, part[1]);
+            part[2] = dfma(r_, r_, part[2]);
+            qq[k] = r_; dd[k] = z_;
+        }
         stv(a.r, qq); stv(a.z, dd);
         return;
     }
-    double qq[U][KF], rr[U][KF], dd[U][KF];
+    double qq[KF], rr[KF], dd[KF];
     ld(a.Ap, qq); ld(a.r, rr); ld(a.d, dd);
     if (s.xupd) {
         // x += alpha_{k-1} p_{k-1}, then x += alpha_k p_k: the same two
         // multiply-adds, in the same order, as one update per iteration
-        double xx[U][KF], pp[U][KF], po[U][KF];
+        double xx[KF], pp[KF], po[KF];
         ld(a.x, xx); ld(s.p_prev, po); ld(s.p, pp);
 #pragma unroll
-        for (int u = 0; u < U; ++u)
-#pragma unroll
-            for (int k = 0; k < KF; ++k)
-                if (k < cnt[u]) xx[u][k] = dfma(s.alpha, pp[u][k], dfma(s.alpha_prev, po[u][k], xx[u][k]));
+        for (int k = 0; k < KF; ++k)
+            if (k < cnt) xx[k] = dfma(s.alpha, pp[k], dfma(s.alpha_prev, po[k], xx[k]));
         stv(a.x, xx);
     }
     const double nalpha = -s.alpha;
 #pragma unroll
-    for (int u = 0; u < U; ++u)
-#pragma unroll
-        for (int k = 0; k < KF; ++k) {
-            if (k >= cnt[u]) continue;
-            double rk = dfma(nalpha, qq[u][k], rr[u][k]);
-            if (s.fi_r && m0[u] + k == s.fi_idx) rk = flipbit(rk, s.fi_bit);
-            rr[u][k] = rk;
-            dd[u][k] = __ddiv_rn(rk, dd[u][k]);          // z
-            part[u][0] = dfma(rk, rk, part[u][0]);
-            part[u][1] = dfma(rk, dd[u][k], part[u][1]);
-        }
+    for (int k = 0; k < KF; ++k) {
+        if (k >= cnt) continue;
+        double rk = dfma(nalpha, qq[k], rr[k]);
+        if (s.fi_r && m0 + k == s.fi_idx) rk = flipbit(rk, s.fi_bit);
+        rr[k] = rk;
+        dd[k] = __ddiv_rn(rk, dd[k]);          // z
+        part[0] = dfma(rk, rk, part[0]);
+        part[1] = dfma(rk, dd[k], part[1]);
+    }
     stv(a.r, rr); stv(a.z, dd);
 }
 
@@ -797,9 +824,8 @@ __global__ void __launch_bounds__(RT, kUpdateCtasPerSm) k_update(UpdateArgs a) {
     // carries one sum through its nodes of all the run's blocks, and the run
     // takes one block tree at the end
     const int G = gridDim.x, c = blockIdx.x;
-    double rp[1][3] = {{0.0, 0.0, 0.0}};
-    for (int blk = c; blk < a.nflat; blk += G) upd_blocks<1, false>(a, us, {blk}, rp);
-    double (&part)[3] = rp[0];
+    double part[3] = {0.0, 0.0, 0.0};
+    for (int blk = c; blk < a.nflat; blk += G) upd_block(a, us, blk, part);
     cta_tree_sum<3>(part, sh);
     if (tid == 0) {
 #pragma unroll

@@ -142,12 +142,21 @@ hs_status sync_state_config(hs_solver* h, int max_iter, double tol) {
 int nblocks(const hs_solver* h) { return (int)h->part.nblk; }
 
 // ---- operator launches -------------------------------------------------------------
+// the operator's instantiation; uniform: rho*c is one value (wht form only);
+// d1: with the checksum
+template <int FORM, bool LOOP>
+const void* slab_kernel(bool uniform, bool d1) {
+    constexpr bool U = FORM == FORM_WHT;
+    if (d1) return uniform && U ? (const void*)k_apply_slab<FORM, LOOP, U, true> : (const void*)k_apply_slab<FORM, LOOP, false, true>;
+    return uniform && U ? (const void*)k_apply_slab<FORM, LOOP, U, false> : (const void*)k_apply_slab<FORM, LOOP, false, false>;
+}
 template <int FORM>
 bool set_smem_form() {
-    return cudaFuncSetAttribute(k_apply_slab<FORM, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)kSlabSmem) == cudaSuccess &&
-           cudaFuncSetAttribute(k_apply_slab<FORM, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)kSlabSmem) == cudaSuccess;
+    bool ok = true;
+    for (int i = 0; i < 4; ++i)
+        for (const void* k : {slab_kernel<FORM, true>(i & 1, i & 2), slab_kernel<FORM, false>(i & 1, i & 2)})
+            ok = ok && cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSlabSmem) == cudaSuccess;
+    return ok;
 }
 bool set_smem_attributes() {
     static bool done = false, ok = true;
@@ -178,9 +187,11 @@ void launch_k(bool pdl, void (*k)(KArgs...), int grid, int block, size_t smem, c
 
 template <int FORM>
 void launch_slab(hs_solver* h, const ApplyArgs& a, bool pdl) {
-    const int g = (int)h->part.ntiles;
-    if (a.role == ROLE_LOOP) launch_k(pdl, k_apply_slab<FORM, true>, g, ST, kSlabSmem, h->s, a);
-    else k_apply_slab<FORM, false><<<g, ST, kSlabSmem, h->s>>>(a);
+    using Kernel = void (*)(ApplyArgs);
+    const bool loop = a.role == ROLE_LOOP;
+    const bool uni = h->rhocmin == h->rhocmax;
+    Kernel k = (Kernel)(loop ? slab_kernel<FORM, true>(uni, a.d1) : slab_kernel<FORM, false>(uni, a.d1));
+    launch_k(pdl && loop, k, (int)h->part.ntiles, ST, kSlabSmem, h->s, a);
 }
 void launch_colored(hs_solver* h, const ApplyArgs& a, bool pdl) {
     switch (h->opt.kernel) {
@@ -213,7 +224,7 @@ ApplyArgs colored_args(hs_solver* h, int role, const double* x, double* y, doubl
     a.part = h->part;
     a.N = h->N; a.role = role; a.dt_eff = dt_eff;
     a.x = x; a.z = h->z.p; a.pbuf0 = h->p0.p; a.pbuf1 = h->p1.p;
-    a.y = y; a.coef = h->coef.p; a.w = w; a.F = F; a.dtF = dtF;
+    a.y = y; a.coef = h->coef.p; a.kc = h->kc.p; a.rc = h->rhocmin; a.w = w; a.F = F; a.dtF = dtF;
     a.d1 = d1 ? 1 : 0;
     a.partials = h->partials.p; a.st = h->st.p; a.ec = h->ec;
     return a;
@@ -381,11 +392,11 @@ hs_status launch_pcg(hs_solver* h, bool with_rhs) {
     HS_CUDA(cudaLaunchCooperativeKernel(pcg_kernel(h, h->coop_grid < a.nruns), dim3(h->coop_grid), dim3(ST), args, pcg_smem(h->part.CX), h->s));
     return HS_OK;
 }
-// a step's iteration count as k_step_end stores it: -1 where the cooperative
-// solve gave up waiting for a CTA
+// a step's iteration count as k_step_end stores it: -1 where a kernel gave up a
+// wait (DevState::stuck)
 hs_status check_iters(const int* it, int n) {
     for (int i = 0; i < n; ++i)
-        if (it[i] < 0) { set_error("the PCG kernel gave up waiting for its other blocks"); return HS_ERR_CUDA; }
+        if (it[i] < 0) { set_error("a kernel gave up waiting for its other warps or blocks"); return HS_ERR_CUDA; }
     return HS_OK;
 }
 
@@ -718,6 +729,7 @@ hs_status hs_apply(hs_solver* s, const double* x, double* y, double dt_eff, int 
     DevState hsx{};
     HS_CUDA(cudaMemcpyAsync(&hsx, s->st.p, sizeof(hsx), cudaMemcpyDeviceToHost, s->s));
     HS_CUDA(cudaStreamSynchronize(s->s));
+    if (hsx.stuck) { const int bad = -1; return check_iters(&bad, 1); }
     if (d1 && abft_rel) *abft_rel = hsx.d1_last;
     return HS_OK;
 }
