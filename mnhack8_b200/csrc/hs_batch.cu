@@ -84,14 +84,14 @@ struct hs_batch {
     std::vector<Slot> slots;
     DevBuf<BInst> d_inst;
     DevBuf<BState> d_st;
-    DevBuf<int> d_t2i, d_f2i;
+    DevBuf<int> d_t2i, d_f2i, d_c2i;
     DevBuf<double> pa, pf;
     DevBuf<double> sq, spart;     // set-up reductions of hs_batch_add
     cudaMemPool_t pool = nullptr; // instance arenas: stream-ordered, kept reserved for reuse
     cudaStream_t s_add = nullptr; // set-up of added instances, overlapping a step in flight
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     bool inflight = false;        // hs_batch_step_begin without its hs_batch_step_end
-    long long cap_tiles = 0, cap_flat = 0;
+    long long cap_tiles = 0, cap_flat = 0, cap_chunk = 0;
     bool dirty = true;            // maps / descriptors need an upload
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t gexec = nullptr;
@@ -114,62 +114,65 @@ void set_bsmem() {
     static bool done = false;
     if (done) return;
     done = true;
-    cudaFuncSetAttribute(kb_apply<double, BK_RESID>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)sizeof(BSlabSmem<double>));
-    cudaFuncSetAttribute(kb_apply<double, BK_RHS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)sizeof(BSlabSmem<double>));
-    cudaFuncSetAttribute(kb_apply<float, BK_LOOP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)sizeof(BSlabSmem<float>));
+    cudaFuncSetAttribute(kb_apply<BK_RESID>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(BSlabSmem));
+    cudaFuncSetAttribute(kb_apply<BK_RHS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(BSlabSmem));
+    cudaFuncSetAttribute(kb_apply32, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(FSlabSmem));
 }
 
 BatchArgs batch_args(hs_batch* b) {
     BatchArgs a{};
-    a.inst = b->d_inst.p; a.tile2inst = b->d_t2i.p; a.flat2inst = b->d_f2i.p;
+    a.inst = b->d_inst.p; a.tile2inst = b->d_t2i.p; a.flat2inst = b->d_f2i.p; a.chunk2inst = b->d_c2i.p;
     a.n_inst = (int)b->slots.size();
-    a.ntiles = b->cap_tiles; a.nflat = b->cap_flat;
+    a.ntiles = b->cap_tiles; a.nflat = b->cap_flat; a.nchunk = b->cap_chunk;
     a.pa = b->pa.p; a.pf = b->pf.p;
     a.rtol = b->opt.rtol; a.inner_tol = b->opt.inner_tol;
     a.max_outer = b->opt.max_outer; a.max_inner = b->opt.max_inner;
     a.detect = b->opt.detect;
     a.extrapolate = b->opt.extrapolate;
+    a.neg0 = 0x8000000080000000ull;
     return a;
 }
 
 // compact the live instances' tile and block ranges; grow the capacity (and
 // drop the graph) when they no longer fit; upload maps and descriptors
 hs_status upload(hs_batch* b) {
-    long long nt = 0, nf = 0;
-    for (auto& sl : b->slots) if (sl.used) { nt += sl.part.ntiles; nf += sl.part.nflat; }
-    if (nt > b->cap_tiles || nf > b->cap_flat || !b->d_t2i.p) {
+    long long nt = 0, nf = 0, nc = 0;
+    for (auto& sl : b->slots) if (sl.used) { nt += sl.part.ntiles; nf += sl.part.nflat; nc += sl.desc.nchunk; }
+    if (nt > b->cap_tiles || nf > b->cap_flat || nc > b->cap_chunk || !b->d_t2i.p) {
         b->cap_tiles = std::max<long long>({nt, 2 * b->cap_tiles, 1024});
         b->cap_flat = std::max<long long>({nf, 2 * b->cap_flat, 1024});
+        // a chunk holds several flat blocks, so there are at most as many
+        b->cap_chunk = std::max<long long>({nc, 2 * b->cap_chunk, 1024 / 4});
         HS_CUDA(b->d_t2i.alloc(b->cap_tiles));
         HS_CUDA(b->d_f2i.alloc(b->cap_flat));
+        HS_CUDA(b->d_c2i.alloc(b->cap_chunk));
         // compensated partials: (hi, lo) per quantity
         HS_CUDA(b->pa.alloc((size_t)2 * MAXQ * b->cap_tiles));
         HS_CUDA(b->pf.alloc((size_t)2 * 4 * b->cap_flat));
         if (b->gexec) { cudaGraphExecDestroy(b->gexec); b->gexec = nullptr; }
         if (b->graph) { cudaGraphDestroy(b->graph); b->graph = nullptr; }
     }
-    std::vector<int> t2i(b->cap_tiles, -1), f2i(b->cap_flat, -1);
+    std::vector<int> t2i(b->cap_tiles, -1), f2i(b->cap_flat, -1), c2i(b->cap_chunk, -1);
     std::vector<BInst> desc(b->slots.size());
-    long long t0 = 0, f0 = 0;
+    long long t0 = 0, f0 = 0, c0 = 0;
     for (size_t i = 0; i < b->slots.size(); ++i) {
         auto& sl = b->slots[i];
         BInst d = sl.desc;
         d.active = 0;
         if (sl.used) {
-            d.tile0 = t0; d.flat0 = f0;
+            d.tile0 = t0; d.flat0 = f0; d.chunk0 = c0;
             for (long long t = 0; t < sl.part.ntiles; ++t) t2i[t0 + t] = (int)i;
             for (long long f = 0; f < sl.part.nflat; ++f) f2i[f0 + f] = (int)i;
-            t0 += sl.part.ntiles; f0 += sl.part.nflat;
+            for (long long c = 0; c < d.nchunk; ++c) c2i[c0 + c] = (int)i;
+            t0 += sl.part.ntiles; f0 += sl.part.nflat; c0 += d.nchunk;
             d.active = sl.steps_left > 0 ? 1 : 0;
         }
-        sl.desc.tile0 = d.tile0; sl.desc.flat0 = d.flat0;
+        sl.desc.tile0 = d.tile0; sl.desc.flat0 = d.flat0; sl.desc.chunk0 = d.chunk0;
         desc[i] = d;
     }
     HS_CUDA(cudaMemcpyAsync(b->d_t2i.p, t2i.data(), t2i.size() * sizeof(int), cudaMemcpyHostToDevice, b->s));
     HS_CUDA(cudaMemcpyAsync(b->d_f2i.p, f2i.data(), f2i.size() * sizeof(int), cudaMemcpyHostToDevice, b->s));
+    HS_CUDA(cudaMemcpyAsync(b->d_c2i.p, c2i.data(), c2i.size() * sizeof(int), cudaMemcpyHostToDevice, b->s));
     HS_CUDA(cudaMemcpyAsync(b->d_inst.p, desc.data(), desc.size() * sizeof(BInst), cudaMemcpyHostToDevice, b->s));
     HS_CUDA(cudaStreamSynchronize(b->s));
     b->dirty = false;
@@ -178,10 +181,16 @@ hs_status upload(hs_batch* b) {
 
 // outer-iteration tail: r = b - A T, test, start of the next inner solve
 void enqueue_resid(hs_batch* b, const BatchArgs& a) {
-    kb_apply<double, BK_RESID><<<(int)a.ntiles, ST, sizeof(BSlabSmem<double>), b->s>>>(a);
+    kb_apply<BK_RESID><<<(int)a.ntiles, ST, sizeof(BSlabSmem), b->s>>>(a);
     kb_final_apply<BK_RESID><<<a.n_inst, RT, 0, b->s>>>(a);
     kb_resid<<<(int)a.nflat, RT, 0, b->s>>>(a);
     kb_outer_final<<<a.n_inst, RT, 0, b->s>>>(a);
+}
+
+// one inner FP32 iteration of every instance still in its inner solve
+void enqueue_inner(hs_batch* b, const BatchArgs& a) {
+    kb_apply32<<<(int)a.ntiles, FT, sizeof(FSlabSmem), b->s>>>(a);
+    kb_update32<<<(int)a.nchunk, RT, 0, b->s>>>(a);
 }
 
 hs_status build_batch_graph(hs_batch* b) {
@@ -195,7 +204,7 @@ hs_status build_batch_graph(hs_batch* b) {
     cudaGraph_t pre;
     HS_CUDA(cudaStreamBeginCapture(b->s, cudaStreamCaptureModeThreadLocal));
     kb_step_begin<<<(a.n_inst + 127) / 128, 128, 0, b->s>>>(a);
-    kb_apply<double, BK_RHS><<<(int)a.ntiles, ST, sizeof(BSlabSmem<double>), b->s>>>(a);
+    kb_apply<BK_RHS><<<(int)a.ntiles, ST, sizeof(BSlabSmem), b->s>>>(a);
     kb_final_apply<BK_RHS><<<a.n_inst, RT, 0, b->s>>>(a);
     kb_extrapolate<<<(int)a.nflat, RT, 0, b->s>>>(a);
     enqueue_resid(b, a);
@@ -232,10 +241,7 @@ hs_status build_batch_graph(hs_batch* b) {
     HS_CUDA(cudaStreamBeginCaptureToGraph(b->s, ibody, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
     // four inner iterations per pass (an instance that is done skips them), one condition
     for (int u = 0; u < 4; ++u) {
-        kb_apply<float, BK_LOOP><<<(int)a.ntiles, ST, sizeof(BSlabSmem<float>), b->s>>>(a);
-        kb_final_apply<BK_LOOP><<<a.n_inst, RT, 0, b->s>>>(a);
-        kb_update32<<<(int)a.nflat, RT, 0, b->s>>>(a);
-        kb_final_update32<<<a.n_inst, RT, 0, b->s>>>(a);
+        enqueue_inner(b, a);
     }
     kb_cond<1><<<1, 1024, 0, b->s>>>(a, c_in, nullptr);
     HS_CUDA(cudaStreamEndCapture(b->s, &ibody));
@@ -268,7 +274,7 @@ hs_status step_direct(hs_batch* b) {
         return HS_OK;
     };
     kb_step_begin<<<(a.n_inst + 127) / 128, 128, 0, b->s>>>(a);
-    kb_apply<double, BK_RHS><<<(int)a.ntiles, ST, sizeof(BSlabSmem<double>), b->s>>>(a);
+    kb_apply<BK_RHS><<<(int)a.ntiles, ST, sizeof(BSlabSmem), b->s>>>(a);
     kb_final_apply<BK_RHS><<<a.n_inst, RT, 0, b->s>>>(a);
     kb_extrapolate<<<(int)a.nflat, RT, 0, b->s>>>(a);
     enqueue_resid(b, a);
@@ -280,10 +286,7 @@ hs_status step_direct(hs_batch* b) {
         for (;;) {
             if (read(1) != HS_OK) return HS_ERR_CUDA;
             if (!host_flag) break;
-            kb_apply<float, BK_LOOP><<<(int)a.ntiles, ST, sizeof(BSlabSmem<float>), b->s>>>(a);
-            kb_final_apply<BK_LOOP><<<a.n_inst, RT, 0, b->s>>>(a);
-            kb_update32<<<(int)a.nflat, RT, 0, b->s>>>(a);
-            kb_final_update32<<<a.n_inst, RT, 0, b->s>>>(a);
+            enqueue_inner(b, a);
             kb_cond<1><<<1, 1024, 0, b->s>>>(a, 0, flag.p + 1);
         }
         kb_correct<<<(int)a.nflat, RT, 0, b->s>>>(a);
@@ -350,9 +353,12 @@ hs_status batch_add_impl(hs_batch* b, int N, double dt, const double* k, const d
                          const double* T0, int n_steps, int* slot_out) {
     HS_CUDA(cudaSetDevice(b->opt.device));
     const long long NN = N + 1, Nn = NN * NN * NN, Ne = (long long)N * N * N;
+    bool uniform = true;            // rho*c is one value
     if (!gen)
-        for (long long e = 0; e < Ne; ++e)
+        for (long long e = 0; e < Ne; ++e) {
             if (!(k[e] > 0) || !(rhoc[e] > 0)) { set_error("hs_batch_add: non-positive coefficient"); return HS_ERR_ARG; }
+            uniform = uniform && rhoc[e] == rhoc[0];
+        }
     const RefMatrices mats = build_reference_matrices(N);
     if (!mats.ok) { set_error("reference-matrix self-check failed"); return HS_ERR_MATRIX; }
     // slot
@@ -419,7 +425,11 @@ hs_status batch_add_impl(hs_batch* b, int N, double dt, const double* k, const d
     }
     if (T0) HS_CUDA(cudaMemcpyAsync(d.T, T0, Nn * 8, cudaMemcpyHostToDevice, sa));
     else HS_CUDA(cudaMemsetAsync(d.T, 0, Nn * 8, sa));
-    k_pack_coef<<<grid_for(Ne, RT), RT, 0, sa>>>(Ne, rh, kk, (double2*)d.coef64, (float2*)d.coef32);
+    d.uniform = uniform ? 1 : 0;
+    d.rc32 = uniform ? (float)(gen ? gen->rhoc : rhoc[0]) : 0.f;
+    d.k32 = (const float*)d.coef32;
+    k_pack_coef<<<grid_for(Ne, RT), RT, 0, sa>>>(Ne, rh, kk, (double2*)d.coef64, (float2*)d.coef32,
+                                                 uniform ? (float*)d.coef32 : nullptr);
     // diagonal, ABFT weights and their norms (node-parallel operator, FP64)
     ElemConsts ec{};
     std::memcpy(ec.M, mats.M, sizeof(ec.M)); std::memcpy(ec.K, mats.K, sizeof(ec.K));
@@ -450,6 +460,7 @@ hs_status batch_add_impl(hs_batch* b, int N, double dt, const double* k, const d
     sl.used = true; sl.N = N; sl.dt = dt; sl.steps_left = n_steps; sl.steps_done = 0;
     sl.part = batch_part(N, b->opt.tile_planes);
     d.part = sl.part;
+    d.nchunk = (Nn + UC - 1) / UC;
     sl.mem = mem;
     sl.desc = d;
     b->dirty = true;

@@ -82,6 +82,8 @@ struct BState {
     int inner_faults;       // inner solves discarded so far
     int has_prev;           // the previous step's field is kept (extrapolated start)
     int extrap;             // this step starts from 2 T - T_prev
+    unsigned tick_a, tick_u;   // blocks of the running inner apply / update that are done
+    int stuck, pad3;        // a bounded wait gave up: the inner solve is discarded
 };
 
 __device__ __forceinline__ float flipf(float x, int bit) {
@@ -96,17 +98,22 @@ __device__ __forceinline__ bool fi_now(const BState* st, int vec) {
 struct BInst {
     Part part;                 // slab tiles and flat blocks of this instance
     long long tile0, flat0;    // first global tile / flat block
+    long long chunk0, nchunk;  // first global chunk of the inner update, and their number
     double dt;
     double cm[4], ck[4];       // wht eigen-constants / 8 of this grid
     float cmf[4], ckf[4];
-    int active, pad;
+    int active;
+    int uniform;               // rho*c is one value: k32 holds k alone
+    float rc32;                // and its value
+    int pad;
     double* T;                 // solution (updated in place)
     double* b;                 // right-hand side M T_old
     double* y64;               // FP64 operator output
     double* r64;               // FP64 residual
     double* Tm1;               // field at the start of the previous step (extrapolated start)
     const double2* coef64;     // (rho*c, k) per element
-    const float2* coef32;
+    const float2* coef32;      // varying rho*c
+    const float* k32;          // uniform rho*c (the same buffer)
     const double* wA;          // ABFT weights A 1_int, M 1_int (FP64)
     const double* wM;
     const float* dinv32;       // 1 / diag, FP32
@@ -123,13 +130,15 @@ struct BatchArgs {
     const BInst* inst;
     const int* tile2inst;      // global tile -> instance slot (-1: none)
     const int* flat2inst;      // global flat block -> instance slot
+    const int* chunk2inst;     // global chunk -> instance slot
     int n_inst, pad;
-    long long ntiles, nflat;   // capacity of the grids
+    long long ntiles, nflat, nchunk;   // capacity of the grids
     double* pa;                // apply partials: [q * ntiles + tile]
     double* pf;                // flat partials:  [q * nflat + block]
     double rtol, inner_tol;
     int max_outer, max_inner;
     int detect, extrapolate;
+    unsigned long long neg0;   // (-0.f, -0.f), see f2_mul
 };
 
 template <typename V> struct VTraits;
@@ -172,30 +181,27 @@ __device__ __forceinline__ void elem_wht_v(V* v, V rhoc, V dk, const V* cm, cons
             if (!(q & bit)) { const V u = v[q], w = v[q | bit]; v[q] = T::add(u, w); v[q | bit] = T::sub(u, w); }
 }
 
-template <typename V>
 struct __align__(16) BSlabSmem {
-    V P[2][SPOS];
-    typename VTraits<V>::V2 Y1[SPOS], Y2[SPOS], Y3[SPOS];
+    double P[2][SPOS];
+    double2 Y1[SPOS], Y2[SPOS], Y3[SPOS];
     double sh[2 * MAXQ][8];
 };
 
-// Batched slab operator.  KIND 0: y64 = A T (FP64, residual); 1: b = M T
-// (FP64, right-hand side); 2: inner FP32 loop, p = z (+ beta p), Ap = A p.
-// Partials per tile: p.Ap (KIND 2), and D1: 1_int.y, w.x, x.x.
-enum BKind { BK_RESID = 0, BK_RHS = 1, BK_LOOP = 2 };
+// Batched slab operator in FP64.  KIND 0: y64 = A T (residual); 1: b = M T
+// (right-hand side).  Partials per tile (compensated): D1's 1_int.y, w.x, x.x.
+enum BKind { BK_RESID = 0, BK_RHS = 1 };
 
-// tile t of instance I; FI false: no vector fault is armed for this launch
-template <typename V, int KIND, bool FI>
-__device__ __forceinline__ void kb_tile(const BatchArgs& B, BSlabSmem<V>& S, long long t, const BInst& I) {
-    using T2 = typename VTraits<V>::V2;
-    using VT = VTraits<V>;
-    BState* st = I.st;
-    const bool loop = KIND == BK_LOOP;
-    if constexpr (KIND == BK_LOOP) {
-        if (st->odone || st->done) return;
-    } else if constexpr (KIND == BK_RESID) {
-        if (st->odone) return;
-    }
+template <int KIND>
+__global__ void __launch_bounds__(ST, 2) kb_apply(BatchArgs B) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    BSlabSmem& S = *reinterpret_cast<BSlabSmem*>(smem_raw);
+    const long long t = blockIdx.x;
+    if (t >= B.ntiles) return;
+    const int slot = B.tile2inst[t];
+    if (slot < 0) return;
+    const BInst& I = B.inst[slot];
+    if (!I.active) return;
+    if (KIND == BK_RESID && I.st->odone) return;
     const Part& P = I.part;
     const int N = P.N, Cw = P.Cw;
     // node and element indices fit in 32 bits (N <= 1200)
@@ -204,67 +210,22 @@ __device__ __forceinline__ void kb_tile(const BatchArgs& B, BSlabSmem<V>& S, lon
     const SlabPos G = slab_pos(P, Tt, threadIdx.x);
     const unsigned fl = G.fl;
     const int tid = threadIdx.x, xa = Tt.xa, xb = Tt.xb;
-    const V dtv = (V)((KIND == BK_RHS) ? 0.0 : I.dt);
-    V cm[4], ck[4];
+    const double dtv = (KIND == BK_RHS) ? 0.0 : I.dt;
+    double cm[4], ck[4];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        cm[j] = (sizeof(V) == 4) ? (V)I.cmf[j] : (V)I.cm[j];
-        ck[j] = (sizeof(V) == 4) ? (V)I.ckf[j] : (V)I.ck[j];
-    }
-    // inputs
-    const int iter = loop ? st->iter : 0;
-    const double betad = loop ? st->beta : 0.0;
-    const V beta = (V)betad;
-    const V* src_a;
-    const V* src_b = nullptr;
-    V* pout = nullptr;
-    V* yout;
-    if constexpr (KIND == BK_LOOP) {
-        src_a = reinterpret_cast<const V*>(I.z32);
-        src_b = (iter > 0) ? reinterpret_cast<const V*>((iter & 1) ? I.p32a : I.p32b) : nullptr;
-        pout = reinterpret_cast<V*>((iter & 1) ? I.p32b : I.p32a);
-        yout = reinterpret_cast<V*>(I.Ap32);
-    } else {
-        src_a = reinterpret_cast<const V*>(I.T);
-        yout = reinterpret_cast<V*>(KIND == BK_RHS ? I.b : I.y64);
-    }
-    const bool two = src_b != nullptr;
+    for (int j = 0; j < 4; ++j) { cm[j] = I.cm[j]; ck[j] = I.ck[j]; }
+    const double* src = I.T;
+    double* yout = KIND == BK_RHS ? I.b : I.y64;
     const double* w = (KIND == BK_RHS) ? I.wM : I.wA;
     const bool d1 = B.detect != 0;
     CSum part[MAXQ] = {{0.0, 0.0}, {0.0, 0.0}, {0.0, 0.0}, {0.0, 0.0}};
 
-    V pA[SK], pB[SK], aA[SK], aB[SK], ra[SK], rb[SK], cr[SK], ckk[SK];
-    double wv[SK];
+    double pA[SK], pB[SK], aA[SK], aB[SK], ra[SK], cr[SK], ckk[SK], wv[SK];
     auto ld_raw = [&](int px) {
         const bool pv = px >= 0 && px <= N;
         const unsigned base = (unsigned)px * plane;
 #pragma unroll
-        for (int k = 0; k < SK; ++k) {
-            const bool v = pv && sp_valid(fl, k);
-            const unsigned n = base + (unsigned)G.noff[k];
-            ra[k] = v ? __ldg(src_a + n) : (V)0;
-            rb[k] = (v && two) ? __ldg(src_b + n) : (V)0;
-        }
-    };
-    int fi_p = 0, fi_ap = 0, fi_bit = 0;
-    long long fi_idx = -1;
-    if constexpr (KIND == BK_LOOP && FI) {
-        fi_p = fi_now(st, FI_P); fi_ap = fi_now(st, FI_AP);
-        fi_bit = st->fi_bit; fi_idx = st->fi_idx;
-    }
-    auto form = [&](V (&p)[SK], int px) {
-#pragma unroll
-        for (int k = 0; k < SK; ++k) p[k] = two ? VT::fma(beta, rb[k], ra[k]) : ra[k];
-        if constexpr (KIND == BK_LOOP && FI) {
-            if (fi_p) {
-#pragma unroll
-                for (int k = 0; k < SK; ++k)
-                    if (sp_valid(fl, k) && (long long)px * plane + G.noff[k] == fi_idx) {
-                        p[k] = flipf(p[k], fi_bit);
-                        st->fi_fired = 1;
-                    }
-            }
-        }
+        for (int k = 0; k < SK; ++k) ra[k] = (pv && sp_valid(fl, k)) ? __ldg(src + (base + (unsigned)G.noff[k])) : 0.0;
     };
     auto ld_coef = [&](int ex) {
         const bool ev = ex >= 0 && ex < N;
@@ -272,14 +233,8 @@ __device__ __forceinline__ void kb_tile(const BatchArgs& B, BSlabSmem<V>& S, lon
 #pragma unroll
         for (int k = 0; k < SK; ++k) {
             const bool v = ev && sp_elem(fl, k);
-            const unsigned e = base + (unsigned)G.eoff[k];
-            if constexpr (sizeof(V) == 4) {
-                const float2 c = v ? __ldg(I.coef32 + e) : make_float2(0.f, 0.f);
-                cr[k] = c.x; ckk[k] = c.y;
-            } else {
-                const double2 c = v ? __ldg(I.coef64 + e) : make_double2(0.0, 0.0);
-                cr[k] = c.x; ckk[k] = c.y;
-            }
+            const double2 c = v ? __ldg(I.coef64 + (base + (unsigned)G.eoff[k])) : make_double2(0.0, 0.0);
+            cr[k] = c.x; ckk[k] = c.y;
         }
     };
     auto ld_w = [&](int px) {
@@ -289,11 +244,10 @@ __device__ __forceinline__ void kb_tile(const BatchArgs& B, BSlabSmem<V>& S, lon
         for (int k = 0; k < SK; ++k)
             wv[k] = (pv && d1 && sp_out(fl, k)) ? __ldg(w + (base + (unsigned)G.noff[k])) : 0.0;
     };
-    auto layer = [&](int ix, int cur, V (&pc)[SK], V (&pn)[SK], V (&ac)[SK], V (&an)[SK]) {
+    auto layer = [&](int ix, int cur, double (&pc)[SK], double (&pn)[SK], double (&ac)[SK], double (&an)[SK]) {
         const int nxt = cur ^ 1;
-        form(pn, ix + 1);
 #pragma unroll
-        for (int k = 0; k < SK; ++k) S.P[nxt][tid + k * ST] = pn[k];
+        for (int k = 0; k < SK; ++k) { pn[k] = ra[k]; S.P[nxt][tid + k * ST] = pn[k]; }
         ld_raw(ix + 2 <= xb + 1 ? ix + 2 : -2);
         __syncthreads();
         if (ix >= 0 && ix < N) {
@@ -301,7 +255,7 @@ __device__ __forceinline__ void kb_tile(const BatchArgs& B, BSlabSmem<V>& S, lon
             for (int k = 0; k < SK; ++k) {
                 if (!sp_elem(fl, k)) continue;
                 const int j = tid + k * ST;
-                V v[8];
+                double v[8];
                 v[0] = pc[k];
                 v[1] = S.P[cur][j + 1];
                 v[2] = S.P[cur][j + Cw];
@@ -310,12 +264,12 @@ __device__ __forceinline__ void kb_tile(const BatchArgs& B, BSlabSmem<V>& S, lon
                 v[5] = S.P[nxt][j + 1];
                 v[6] = S.P[nxt][j + Cw];
                 v[7] = S.P[nxt][j + Cw + 1];
-                elem_wht_v<V>(v, cr[k], VT::mul(dtv, ckk[k]), cm, ck);
-                ac[k] = VT::add(ac[k], v[0]);
-                an[k] = VT::add((V)0, v[4]);
-                S.Y1[j + 1] = T2{v[1], v[5]};
-                S.Y2[j + Cw] = T2{v[2], v[6]};
-                S.Y3[j + Cw + 1] = T2{v[3], v[7]};
+                elem_wht_v<double>(v, cr[k], dmul(dtv, ckk[k]), cm, ck);
+                ac[k] = dadd(ac[k], v[0]);
+                an[k] = dadd(0.0, v[4]);
+                S.Y1[j + 1] = make_double2(v[1], v[5]);
+                S.Y2[j + Cw] = make_double2(v[2], v[6]);
+                S.Y3[j + Cw + 1] = make_double2(v[3], v[7]);
             }
         }
         ld_coef(ix + 1 <= xb ? ix + 1 : -1);
@@ -327,45 +281,26 @@ __device__ __forceinline__ void kb_tile(const BatchArgs& B, BSlabSmem<V>& S, lon
             if (!sp_out(fl, k)) continue;
             const int j = tid + k * ST;
             const bool yzin = !sp_yzb(fl, k);
-            T2 y3{(V)0, (V)0}, y2 = y3, y1 = y3;
+            double2 y3 = make_double2(0.0, 0.0), y2 = y3, y1 = y3;
             if (yzin) { y3 = S.Y3[j]; y2 = S.Y2[j]; y1 = S.Y1[j]; }
             if (ix >= xa) {
                 const unsigned n = base + (unsigned)G.noff[k];
                 const bool bnd = !yzin || xbnd;
-                V y = bnd ? (V)0 : VT::add(VT::add(VT::add(ac[k], y3.x), y2.x), y1.x);
-                if constexpr (KIND == BK_LOOP && FI) {
-                    if (fi_ap && (long long)n == fi_idx) { y = flipf(y, fi_bit); st->fi_fired = 1; }
-                }
-                const double pv = (double)pc[k], yd = (double)y;
-                if constexpr (sizeof(V) == 8) {
-                    // FP64 applies (right-hand side, outer residual): compensated sums
-                    if (loop) csum_fma(part[0], pv, yd);
-                    if (d1) {
-                        if (!bnd) csum_add(part[1], yd);
-                        csum_fma(part[2], wv[k], pv);
-                        part[3].hi = dfma(pv, pv, part[3].hi);  // the norm only scales the threshold
-                    }
-                } else {
-                    // FP32 inner applies: FP64 sums of FP32 values; their rounding (~1e-16 n)
-                    // is far below the FP32 operator's own (~1e-9), so no compensation
-                    if (loop) part[0].hi = dfma(pv, yd, part[0].hi);
-                    if (d1) {
-                        if (!bnd) part[1].hi = dadd(part[1].hi, yd);
-                        part[2].hi = dfma(wv[k], pv, part[2].hi);
-                        part[3].hi = dfma(pv, pv, part[3].hi);
-                    }
+                const double y = bnd ? 0.0 : dadd(dadd(dadd(ac[k], y3.x), y2.x), y1.x);
+                if (d1) {
+                    if (!bnd) csum_add(part[1], y);
+                    csum_fma(part[2], wv[k], pc[k]);
+                    part[3].hi = dfma(pc[k], pc[k], part[3].hi);  // the norm only scales the threshold
                 }
                 __stwb(yout + n, y);                      // global stores (the pointers come from global memory)
-                if (loop) __stwb(pout + n, pc[k]);
             }
-            an[k] = yzin ? VT::add(VT::add(VT::add(an[k], y3.y), y2.y), y1.y) : (V)0;
+            an[k] = yzin ? dadd(dadd(dadd(an[k], y3.y), y2.y), y1.y) : 0.0;
         }
         ld_w(ix + 1);
     };
     ld_raw(xa - 1);
-    form(pA, xa - 1);
 #pragma unroll
-    for (int k = 0; k < SK; ++k) { S.P[0][tid + k * ST] = pA[k]; aA[k] = (V)0; aB[k] = (V)0; }
+    for (int k = 0; k < SK; ++k) { pA[k] = ra[k]; S.P[0][tid + k * ST] = pA[k]; aA[k] = 0.0; aB[k] = 0.0; }
     ld_raw(xa);
     ld_coef(xa - 1);
     for (int ix = xa - 1; ix <= xb; ++ix) {
@@ -373,37 +308,367 @@ __device__ __forceinline__ void kb_tile(const BatchArgs& B, BSlabSmem<V>& S, lon
 #pragma unroll
         for (int k = 0; k < SK; ++k) { pA[k] = pB[k]; aA[k] = aB[k]; }
     }
-    if (!loop && !d1) return;
-    if constexpr (sizeof(V) == 8) {
-        cta_tree_csum<MAXQ>(part, S.sh);
-        if (threadIdx.x == 0) store_cpartials<MAXQ>(part, B.pa, B.ntiles, t);
-    } else {
-        // FP32 applies: plain FP64 sums, stored with lo = 0 in the same layout
-        double ph[MAXQ] = {part[0].hi, part[1].hi, part[2].hi, part[3].hi};
-        cta_tree_sum<MAXQ>(ph, S.sh);
-        if (threadIdx.x == 0) {
-            const CSum pc[MAXQ] = {{ph[0], 0.0}, {ph[1], 0.0}, {ph[2], 0.0}, {ph[3], 0.0}};
-            store_cpartials<MAXQ>(pc, B.pa, B.ntiles, t);
+    if (!d1) return;
+    cta_tree_csum<MAXQ>(part, S.sh);
+    if (threadIdx.x == 0) store_cpartials<MAXQ>(part, B.pa, B.ntiles, t);
+}
+
+__device__ __forceinline__ double d1_rel(const double (&p)[MAXQ], double nw) {
+    const double nx = __dsqrt_rn(p[3]);
+    double rel = __ddiv_rn(fabs(dsub(p[1], p[2])), dfma(nw, nx, 1e-300));
+    if (!isfinite(rel)) rel = 1e300;
+    return rel;
+}
+
+// ---- the FP32 inner loop: operator ------------------------------------------------
+// The slab march of the FP64 operator (k_apply_slab: one barrier per layer,
+// p stored and checked as it is formed) in FP32: a thread applies its FK
+// elements two at a time in packed FP32 registers, and uniform rho*c is read as
+// one value.  The FP64 sums of the FP32 products (p.Ap, 1_int.Ap, w.p, p.p) are
+// per thread, per tile (a block tree), and then per instance by the last CTA of
+// the instance to finish (an atomic ticket), which also sets alpha; a launch
+// per iteration did that before.
+//
+// Bound by issue and latency (N=160: 54 us, IPC 0.55 a scheduler, against 20 us
+// of HBM traffic).  Measured (B200, device ms of all steps; two barriers a layer,
+// separate final kernels -> this): 24 instances of N 16..96, 20 steps 158.8 ->
+// 148; N=160, 10 steps 162.6 -> 148, of which the packed arithmetic 153 -> 148.  Slower: 512 threads of two
+// positions (64 registers: spills, 158 and 162), three or four CTAs per SM (169
+// and 193, 215 and 298), inputs two layers ahead (164 and 170).
+constexpr int FT = 256, FK = SPOS / FT;
+struct __align__(16) FSlabSmem {
+    float P[3][SPOS];
+    float2 Y1[SPOS], Y2[SPOS], Y3[SPOS];
+    double sh[MAXQ][16];
+    unsigned long long free_bar;
+    unsigned last;
+};
+
+// sum over a CTA of W warps: xor butterfly per warp, then over the warp sums;
+// valid in thread 0
+template <int NQ, int W>
+__device__ __forceinline__ void cta_tree_w(double (&v)[NQ], double (*sh)[16]) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int off = 16; off >= 1; off >>= 1)
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) v[q] = dadd(v[q], __shfl_xor_sync(0xffffffffu, v[q], off));
+    __syncthreads();
+    if (lane == 0) {
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) sh[q][warp] = v[q];
+    }
+    __syncthreads();
+    if (warp == 0) {
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) v[q] = sh[q][lane % W];
+#pragma unroll
+        for (int off = W / 2; off >= 1; off >>= 1)
+#pragma unroll
+            for (int q = 0; q < NQ; ++q) v[q] = dadd(v[q], __shfl_xor_sync(0xffffffffu, v[q], off));
+    }
+}
+// The CTA's sums become partial idx of an instance's count partials (quantity q
+// at base + q * stride); in the last CTA to get here they are added up (strided
+// sums, then the tree) and true is returned, with the totals in thread 0.
+template <int NQ, int NT, int FB>
+__device__ __forceinline__ bool inst_finish(double (&v)[NQ], double* base, long long stride, long long idx,
+                                            long long count, unsigned* ticket, double (*sh)[16], unsigned* s_last) {
+    cta_tree_w<NQ, NT / 32>(v, sh);
+    if (threadIdx.x == 0) {
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) base[q * stride + idx] = v[q];
+        __threadfence();
+        *s_last = atomicAdd(ticket, 1u) == (unsigned)(count - 1) ? 1u : 0u;
+    }
+    __syncthreads();
+    if (!*s_last) return false;
+    __threadfence();
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) v[q] = 0.0;
+    for (long long k0 = threadIdx.x; k0 < count; k0 += (long long)NT * FB) {
+        double t[NQ][FB];
+#pragma unroll
+        for (int q = 0; q < NQ; ++q)
+#pragma unroll
+            for (int u = 0; u < FB; ++u) {
+                const long long k = k0 + (long long)u * NT;
+                t[q][u] = k < count ? __ldcg(base + q * stride + k) : 0.0;
+            }
+#pragma unroll
+        for (int q = 0; q < NQ; ++q)
+#pragma unroll
+            for (int u = 0; u < FB; ++u) v[q] = dadd(v[q], t[q][u]);
+    }
+    cta_tree_w<NQ, NT / 32>(v, sh);
+    if (threadIdx.x == 0) *ticket = 0u;
+    return true;
+}
+
+// Two FP32 lanes in one 64-bit register, each rounded like the scalar operation.
+typedef unsigned long long F2;
+__device__ __forceinline__ F2 f2(float lo, float hi) {
+    F2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ void f2_get(F2 v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
+__device__ __forceinline__ F2 f2_add(F2 a, F2 b) { F2 r; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
+__device__ __forceinline__ F2 f2_sub(F2 a, F2 b) { F2 r; asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
+// A product as a multiply-add of -0, which the caller passes as a run-time
+// value: the assembler contracts mul.rn.f32x2, and a multiply-add of a constant
+// -0, with the addition that follows (seen on sm_100a with CUDA 12.9 despite
+// --fmad=false; it changes the result's last bit).
+__device__ __forceinline__ F2 f2_mul(F2 a, F2 b, F2 neg0) {
+    F2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(neg0));
+    return r;
+}
+__device__ __forceinline__ F2 f2_fma(F2 a, F2 b, F2 c) { F2 r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c)); return r; }
+// elem_wht_v on two elements side by side
+__device__ __forceinline__ void elem_wht_f2(F2* v, F2 rhoc, F2 dk, const float* cm, const float* ck, F2 neg0) {
+#pragma unroll
+    for (int bit = 1; bit <= 4; bit <<= 1)
+#pragma unroll
+        for (int q = 0; q < 8; ++q)
+            if (!(q & bit)) { const F2 u = v[q], w = v[q | bit]; v[q] = f2_add(u, w); v[q | bit] = f2_sub(u, w); }
+    const F2 l0 = f2_mul(rhoc, f2(cm[0], cm[0]), neg0);
+    F2 l[4];
+#pragma unroll
+    for (int j = 1; j < 4; ++j) l[j] = f2_fma(dk, f2(ck[j], ck[j]), f2_mul(rhoc, f2(cm[j], cm[j]), neg0));
+    v[0] = f2_mul(v[0], l0, neg0);
+    v[1] = f2_mul(v[1], l[1], neg0); v[2] = f2_mul(v[2], l[1], neg0); v[4] = f2_mul(v[4], l[1], neg0);
+    v[3] = f2_mul(v[3], l[2], neg0); v[5] = f2_mul(v[5], l[2], neg0); v[6] = f2_mul(v[6], l[2], neg0);
+    v[7] = f2_mul(v[7], l[3], neg0);
+#pragma unroll
+    for (int bit = 1; bit <= 4; bit <<= 1)
+#pragma unroll
+        for (int q = 0; q < 8; ++q)
+            if (!(q & bit)) { const F2 u = v[q], w = v[q | bit]; v[q] = f2_add(u, w); v[q | bit] = f2_sub(u, w); }
+}
+
+// RC: uniform rho*c.  FI: an armed flip of p or Ap fires in this iteration.
+template <bool RC, bool FI>
+__device__ __forceinline__ void kb_march32(const BatchArgs& B, FSlabSmem& S, const BInst& I, const SlabTile& T,
+                                           double (&part)[MAXQ]) {
+    using VT = VTraits<float>;
+    BState* st = I.st;
+    const Part& P = I.part;
+    const int N = P.N, Cw = P.Cw, npos = P.Rw * P.Cw;
+    const unsigned plane = (unsigned)P.NN * (unsigned)P.NN, eplane = (unsigned)N * (unsigned)N;
+    const int tid = threadIdx.x, lane = tid & 31, xa = T.xa, xb = T.xb;
+    // geometry (slab_pos with FT threads): node and element offsets, flags as there
+    unsigned noff[FK], eoff[FK], fl = 0u;
+    bool on[FK];                                    // some position of this warp's k-th row exists
+#pragma unroll
+    for (int k = 0; k < FK; ++k) {
+        const int j = tid + k * FT;
+        const int lr = j / Cw, lc = j - lr * Cw, gy = T.y0 - 1 + lr, gz = T.z0 - 1 + lc;
+        const bool in = j < npos;
+        const bool valid = in && gy >= 0 && gy <= N && gz >= 0 && gz <= N;
+        const bool elem = in && lr <= P.Rw - 2 && lc <= Cw - 2 && gy >= 0 && gy < N && gz >= 0 && gz < N;
+        const bool out = valid && lr >= 1 && lr <= P.Rw - 2 && lc >= 1 && lc <= Cw - 2;
+        const bool yzb = gy == 0 || gy == N || gz == 0 || gz == N;
+        noff[k] = valid ? (unsigned)(gy * P.NN + gz) : 0u;
+        eoff[k] = elem ? (unsigned)(gy * N + gz) : 0u;
+        fl |= (valid ? 1u : 0u) << k | (elem ? 1u : 0u) << (8 + k) | (out ? 1u : 0u) << (16 + k) |
+              (yzb ? 1u : 0u) << (24 + k);
+        on[k] = (j & ~31) < npos;
+    }
+    const float dtv = (float)I.dt, rc = RC ? I.rc32 : 0.f;
+    float cm[4], ck[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) { cm[j] = I.cmf[j]; ck[j] = I.ckf[j]; }
+    const int iter = st->iter;
+    const float beta = (float)st->beta;
+    const float* src_a = I.z32;
+    const bool two = iter > 0;
+    const float* src_b = two ? ((iter & 1) ? I.p32a : I.p32b) : src_a;
+    float* pout = (iter & 1) ? I.p32b : I.p32a;
+    float* yout = I.Ap32;
+    const double* w = I.wA;
+    const bool d1 = B.detect != 0;
+    const bool fi_p = FI && fi_now(st, FI_P), fi_ap = FI && fi_now(st, FI_AP);
+    const int fi_bit = FI ? st->fi_bit : 0;
+    const long long fi_idx = FI ? st->fi_idx : -1;
+
+    float cr[FK], ckk[FK];
+    auto ld_raw = [&](int px, float (&ra)[FK], float (&rb)[FK], double (&wv)[FK]) {
+        const bool pv = px >= 0 && px <= N, pt = px >= xa && px <= xb;
+        const unsigned base = (unsigned)px * plane;
+#pragma unroll
+        for (int k = 0; k < FK; ++k) {
+            const bool v = pv && sp_valid(fl, k);
+            const unsigned n = base + noff[k];
+            ra[k] = v ? __ldg(src_a + n) : 0.f;
+            rb[k] = (v && two) ? __ldg(src_b + n) : 0.f;
+            wv[k] = (pt && d1 && sp_out(fl, k)) ? __ldg(w + n) : 0.0;
         }
+    };
+    auto form = [&](int px, float* Pl, const float (&ra)[FK], const float (&rb)[FK], const double (&wv)[FK]) {
+        const bool pt = px >= xa && px <= xb;
+        const unsigned base = (unsigned)px * plane;
+#pragma unroll
+        for (int k = 0; k < FK; ++k) {
+            float v = two ? VT::fma(beta, rb[k], ra[k]) : ra[k];
+            if (fi_p && sp_valid(fl, k) && (long long)px * plane + noff[k] == fi_idx) {
+                v = flipf(v, fi_bit);
+                st->fi_fired = 1;
+            }
+            Pl[tid + k * FT] = v;
+            if (pt && sp_out(fl, k)) {
+                if (d1) {
+                    const double vd = (double)v;
+                    part[2] = dfma(wv[k], vd, part[2]);
+                    part[3] = dfma(vd, vd, part[3]);
+                }
+                __stwb(pout + (base + noff[k]), v);        // global stores (the pointers come from global memory)
+            }
+        }
+    };
+    auto ld_coef = [&](int ex) {
+        const bool ev = ex >= 0 && ex < N;
+        const unsigned base = (unsigned)ex * eplane;
+#pragma unroll
+        for (int k = 0; k < FK; ++k) {
+            const bool v = ev && sp_elem(fl, k);
+            if constexpr (RC) {
+                ckk[k] = v ? __ldg(I.k32 + (base + eoff[k])) : 0.f;
+            } else {
+                const float2 c = v ? __ldg(I.coef32 + (base + eoff[k])) : make_float2(0.f, 0.f);
+                cr[k] = c.x; ckk[k] = c.y;
+            }
+        }
+    };
+    const unsigned free_bar = (unsigned)__cvta_generic_to_shared(&S.free_bar);
+    unsigned phase = 0;
+    float ac[FK], an[FK], ra[FK], rb[FK];
+    double wv[FK];
+    auto layer = [&](int ix, float* P0, float* P1, float* P2) {
+        const bool el = ix >= 0 && ix < N;
+#pragma unroll
+        for (int k = 0; k < FK; k += 2) {
+            an[k] = an[k + 1] = 0.f;
+            F2 v[8];
+            const int j = tid + k * FT, i = j + FT;
+            if (el && on[k]) {
+                v[0] = f2(P0[j], P0[i]);
+                v[1] = f2(P0[j + 1], P0[i + 1]);
+                v[2] = f2(P0[j + Cw], P0[i + Cw]);
+                v[3] = f2(P0[j + Cw + 1], P0[i + Cw + 1]);
+                v[4] = f2(P1[j], P1[i]);
+                v[5] = f2(P1[j + 1], P1[i + 1]);
+                v[6] = f2(P1[j + Cw], P1[i + Cw]);
+                v[7] = f2(P1[j + Cw + 1], P1[i + Cw + 1]);
+                elem_wht_f2(v, RC ? f2(rc, rc) : f2(cr[k], cr[k + 1]), f2(VT::mul(dtv, ckk[k]), VT::mul(dtv, ckk[k + 1])),
+                            cm, ck, B.neg0);
+                float a, b;
+                f2_get(v[0], a, b);
+                ac[k] = VT::add(ac[k], a); ac[k + 1] = VT::add(ac[k + 1], b);
+                f2_get(v[4], a, b);
+                an[k] = VT::add(0.f, a); an[k + 1] = VT::add(0.f, b);
+            }
+            // the hand-over buffers are free again
+            if (k == 0 && ix >= xa && !mbar_wait(free_bar, phase)) st->stuck = 1;
+            if (el) {
+                float a[8], b[8];
+#pragma unroll
+                for (int q = 1; q < 8; ++q) f2_get(v[q], a[q], b[q]);
+                if (sp_elem(fl, k)) {
+                    S.Y1[j + 1] = make_float2(a[1], a[5]);
+                    S.Y2[j + Cw] = make_float2(a[2], a[6]);
+                    S.Y3[j + Cw + 1] = make_float2(a[3], a[7]);
+                }
+                if (sp_elem(fl, k + 1)) {
+                    S.Y1[i + 1] = make_float2(b[1], b[5]);
+                    S.Y2[i + Cw] = make_float2(b[2], b[6]);
+                    S.Y3[i + Cw + 1] = make_float2(b[3], b[7]);
+                }
+            }
+        }
+        if (ix >= xa) phase ^= 1u;
+        ld_coef(ix + 1 <= xb ? ix + 1 : -1);
+        form(ix + 2, P2, ra, rb, wv);
+        ld_raw(ix + 3 <= xb + 1 ? ix + 3 : -2, ra, rb, wv);
+        __syncthreads();
+        const unsigned base = (unsigned)ix * plane;
+        const bool xbnd = ix == 0 || ix == N;
+#pragma unroll
+        for (int k = 0; k < FK; ++k) {
+            if (!sp_out(fl, k)) continue;
+            const int j = tid + k * FT;
+            const bool yzin = !sp_yzb(fl, k);
+            float2 y3 = make_float2(0.f, 0.f), y2 = y3, y1 = y3;
+            if (yzin) { y3 = S.Y3[j]; y2 = S.Y2[j]; y1 = S.Y1[j]; }
+            if (ix >= xa) {
+                const unsigned n = base + noff[k];
+                const bool bnd = !yzin || xbnd;
+                float y = bnd ? 0.f : VT::add(VT::add(VT::add(ac[k], y3.x), y2.x), y1.x);
+                if (fi_ap && (long long)n == fi_idx) { y = flipf(y, fi_bit); st->fi_fired = 1; }
+                const double yd = (double)y;
+                part[0] = dfma((double)P0[j], yd, part[0]);
+                if (d1 && !bnd) part[1] = dadd(part[1], yd);
+                __stwb(yout + n, y);
+            }
+            ac[k] = yzin ? VT::add(VT::add(VT::add(an[k], y3.y), y2.y), y1.y) : 0.f;
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(free_bar);
+    };
+    if (tid == 0) mbar_init(free_bar, FT / 32);
+    float *P0 = S.P[0], *P1 = S.P[1], *P2 = S.P[2];
+    {
+        float ra0[FK], rb0[FK];
+        double wv0[FK];
+        ld_raw(xa - 1, ra0, rb0, wv0);
+        ld_raw(xa, ra, rb, wv);
+        ld_coef(xa - 1);
+#pragma unroll
+        for (int k = 0; k < FK; ++k) ac[k] = 0.f;
+        form(xa - 1, P0, ra0, rb0, wv0);
+        form(xa, P1, ra, rb, wv);
+        ld_raw(xa + 1, ra, rb, wv);
+    }
+    __syncthreads();
+    for (int ix = xa - 1; ix <= xb; ++ix) {
+        layer(ix, P0, P1, P2);
+        float* t = P0; P0 = P1; P1 = P2; P2 = t;
     }
 }
 
-template <typename V, int KIND>
-__global__ void __launch_bounds__(ST, 2) kb_apply(BatchArgs B) {
+// p = z + beta p, Ap = A p on every tile; per instance p.Ap -> alpha and the FP32 checksum
+__global__ void __launch_bounds__(FT, 2) kb_apply32(BatchArgs B) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    BSlabSmem<V>& S = *reinterpret_cast<BSlabSmem<V>*>(smem_raw);
+    FSlabSmem& S = *reinterpret_cast<FSlabSmem*>(smem_raw);
     const long long t = blockIdx.x;
-    if (t >= B.ntiles) return;
     const int slot = B.tile2inst[t];
     if (slot < 0) return;
     const BInst& I = B.inst[slot];
     if (!I.active) return;
-    if constexpr (KIND == BK_LOOP) {
-        if (fi_now(I.st, FI_P) || fi_now(I.st, FI_AP)) kb_tile<V, KIND, true>(B, S, t, I);
-        else kb_tile<V, KIND, false>(B, S, t, I);
+    BState* st = I.st;
+    if (st->odone || st->done) return;
+    const SlabTile T = slab_tile(I.part, t - I.tile0);
+    double part[MAXQ] = {0.0, 0.0, 0.0, 0.0};
+    const bool fi = fi_now(st, FI_P) || fi_now(st, FI_AP);
+    if (I.uniform) {
+        if (fi) kb_march32<true, true>(B, S, I, T, part);
+        else kb_march32<true, false>(B, S, I, T, part);
     } else {
-        kb_tile<V, KIND, false>(B, S, t, I);
+        if (fi) kb_march32<false, true>(B, S, I, T, part);
+        else kb_march32<false, false>(B, S, I, T, part);
     }
+    const long long nt = I.part.ntiles;
+    if (!inst_finish<MAXQ, FT, 2>(part, B.pa + I.tile0, B.ntiles, t - I.tile0, nt, &st->tick_a, S.sh, &S.last)) return;
+    if (threadIdx.x != 0) return;
+    if (B.detect) {
+        const double rel = d1_rel(part, st->norm_wA);
+        st->d1_last = rel;
+        st->d1_max32 = fmax(st->d1_max32, rel);
+    }
+    st->applies32 += 1;
+    if (!isfinite(part[0]) || st->stuck) { st->inner_bad = 1; st->done = 1; st->stuck = 0; }
+    else if (fabs(part[0]) < 1e-30) { st->broken = 1; st->done = 1; }
+    else st->alpha = __ddiv_rn(st->rho, part[0]);
 }
 
 // compensated sums of one instance's partials: count (hi, lo) pairs per
@@ -437,41 +702,7 @@ __device__ __forceinline__ void inst_sums(double (&v)[NQ], const double* base, l
     for (int q = 0; q < NQ; ++q) v[q] = csum_value(acc[q]);
 }
 
-// plain sums of one instance's partials whose lo parts are zero (the FP32
-// inner solve's): hi of quantity q at base + q*qstride; RT strided sequential
-// sums, then the block tree; valid in thread 0
-template <int NQ>
-__device__ __forceinline__ void inst_sums_plain(double (&v)[NQ], const double* base, long long count,
-                                                long long qstride, double (*sh)[8]) {
-    constexpr int FB = 8;
-#pragma unroll
-    for (int q = 0; q < NQ; ++q) v[q] = 0.0;
-    for (long long k0 = threadIdx.x; k0 < count; k0 += (long long)RT * FB) {
-        double th[NQ][FB];
-#pragma unroll
-        for (int q = 0; q < NQ; ++q)
-#pragma unroll
-            for (int u = 0; u < FB; ++u) {
-                const long long k = k0 + (long long)u * RT;
-                th[q][u] = (k < count) ? __ldcg(base + q * qstride + k) : 0.0;
-            }
-#pragma unroll
-        for (int q = 0; q < NQ; ++q)
-#pragma unroll
-            for (int u = 0; u < FB; ++u)
-                if (k0 + (long long)u * RT < count) v[q] = dadd(v[q], th[q][u]);
-    }
-    cta_tree_sum<NQ>(v, sh);
-}
-
-__device__ __forceinline__ double d1_rel(const double (&p)[MAXQ], double nw) {
-    const double nx = __dsqrt_rn(p[3]);
-    double rel = __ddiv_rn(fabs(dsub(p[1], p[2])), dfma(nw, nx, 1e-300));
-    if (!isfinite(rel)) rel = 1e300;
-    return rel;
-}
-
-// one block per instance: operator partials -> D1 (and alpha in the loop)
+// one block per instance: an FP64 apply's partials -> D1
 template <int KIND>
 __global__ void __launch_bounds__(RT) kb_final_apply(BatchArgs B) {
     __shared__ double sh[2 * MAXQ][8];
@@ -480,26 +711,16 @@ __global__ void __launch_bounds__(RT) kb_final_apply(BatchArgs B) {
     const BInst& I = B.inst[slot];
     if (!I.active) return;
     BState* st = I.st;
-    if (KIND == BK_LOOP && (st->odone || st->done)) return;
     if (KIND == BK_RESID && st->odone) return;
     double p[MAXQ];
-    if (KIND == BK_LOOP) inst_sums_plain<MAXQ>(p, B.pa + I.tile0, I.part.ntiles, B.ntiles, sh);
-    else inst_sums<MAXQ>(p, B.pa + I.tile0, I.part.ntiles, B.ntiles, sh);
+    inst_sums<MAXQ>(p, B.pa + I.tile0, I.part.ntiles, B.ntiles, sh);
     if (threadIdx.x != 0) return;
     if (B.detect) {
         const double rel = d1_rel(p, KIND == BK_RHS ? st->norm_wM : st->norm_wA);
         st->d1_last = rel;
-        if (KIND == BK_LOOP) st->d1_max32 = fmax(st->d1_max32, rel);
-        else st->d1_max64 = fmax(st->d1_max64, rel);
+        st->d1_max64 = fmax(st->d1_max64, rel);
     }
-    if (KIND == BK_LOOP) {
-        st->applies32 += 1;
-        if (!isfinite(p[0])) { st->inner_bad = 1; st->done = 1; }
-        else if (fabs(p[0]) < 1e-30) { st->broken = 1; st->done = 1; }
-        else st->alpha = __ddiv_rn(st->rho, p[0]);
-    } else {
-        st->applies64 += 1;
-    }
+    st->applies64 += 1;
 }
 
 // flat block of an instance: slot, local block, first node, node count (0..KF)
@@ -582,89 +803,74 @@ __global__ void __launch_bounds__(RT) kb_outer_final(BatchArgs B) {
     if (!isfinite(st->bn_in) || !isfinite(p[2])) st->inner_bad = 1;
 }
 
-// inner FP32 update: d += alpha p, r -= alpha Ap, z = r / diag; partials r.r, r.z
+// ---- the FP32 inner loop: vector update ----------------------------------------------
+// d += alpha p, r -= alpha Ap, z = r / diag; r.r and r.z.  A block takes a chunk
+// of UC consecutive nodes, UV groups of four per thread with every load in
+// flight at once; the last block of an instance to finish adds up its chunks'
+// sums and does the inner solve's scalar step (beta, convergence).
+constexpr int UV = 2, UC = RT * 4 * UV;
 __global__ void __launch_bounds__(RT) kb_update32(BatchArgs B) {
-    __shared__ double sh[2 * MAXQ][8];
-    const FlatPos f = flat_pos(B);
-    CSum part[2] = {{0.0, 0.0}, {0.0, 0.0}};
-    if (f.slot >= 0) {
-        const BInst& I = B.inst[f.slot];
-        const BState* st = I.st;
-        if (I.active && !st->odone && !st->done) {
-            const int iter = st->iter;
-            const float alpha = (float)st->alpha;
-            const float* p = (iter & 1) ? I.p32b : I.p32a;
-            const bool fr = fi_now(st, FI_RV);
-            // the thread's node pair as 8-byte vectors (m0 is even, the buffers 256-byte aligned)
-            float dv[2], pv[2], qv[2], rv[2], iv[2];
-            if (f.cnt == 2) {
-                const float2 a = *reinterpret_cast<const float2*>(I.d32 + f.m0);
-                const float2 b = *reinterpret_cast<const float2*>(p + f.m0);
-                const float2 c = *reinterpret_cast<const float2*>(I.Ap32 + f.m0);
-                const float2 d = *reinterpret_cast<const float2*>(I.r32 + f.m0);
-                const float2 e = __ldg(reinterpret_cast<const float2*>(I.dinv32 + f.m0));
-                dv[0] = a.x; dv[1] = a.y; pv[0] = b.x; pv[1] = b.y; qv[0] = c.x; qv[1] = c.y;
-                rv[0] = d.x; rv[1] = d.y; iv[0] = e.x; iv[1] = e.y;
-            } else {
-                for (int k = 0; k < 2; ++k) {
-                    const bool in = k < f.cnt;
-                    const long long m = f.m0 + k;
-                    dv[k] = in ? I.d32[m] : 0.f; pv[k] = in ? p[m] : 0.f; qv[k] = in ? I.Ap32[m] : 0.f;
-                    rv[k] = in ? I.r32[m] : 0.f; iv[k] = in ? I.dinv32[m] : 0.f;
-                }
-            }
-            float zv[2];
-#pragma unroll
-            for (int k = 0; k < 2; ++k) {
-                dv[k] = __fmaf_rn(alpha, pv[k], dv[k]);
-                float r = __fmaf_rn(-alpha, qv[k], rv[k]);
-                if (fr && f.m0 + k == st->fi_idx && k < f.cnt) { r = flipf(r, st->fi_bit); I.st->fi_fired = 1; }
-                rv[k] = r;
-                zv[k] = __fmul_rn(r, iv[k]);
-                if (k < f.cnt) {
-                    // products of FP32 values are exact in FP64; plain FP64 sums suffice
-                    // for the inner solve's 1e-4 relative tolerance
-                    part[0].hi = dfma((double)r, (double)r, part[0].hi);
-                    part[1].hi = dfma((double)r, (double)zv[k], part[1].hi);
-                }
-            }
-            if (f.cnt == 2) {
-                *reinterpret_cast<float2*>(I.d32 + f.m0) = make_float2(dv[0], dv[1]);
-                *reinterpret_cast<float2*>(I.r32 + f.m0) = make_float2(rv[0], rv[1]);
-                *reinterpret_cast<float2*>(I.z32 + f.m0) = make_float2(zv[0], zv[1]);
-            } else if (f.cnt == 1) {
-                I.d32[f.m0] = dv[0]; I.r32[f.m0] = rv[0]; I.z32[f.m0] = zv[0];
-            }
-        }
-    }
-    // plain FP64 block tree (the inner sums carry no compensation); the
-    // partials keep the (hi, lo) layout of the compensated ones, lo = 0
-    double ph[2] = {part[0].hi, part[1].hi};
-    cta_tree_sum<2>(ph, sh);
-    if (threadIdx.x == 0 && blockIdx.x < B.nflat) {
-        const CSum pc[2] = {{ph[0], 0.0}, {ph[1], 0.0}};
-        store_cpartials<2>(pc, B.pf, B.nflat, blockIdx.x);
-    }
-}
-
-// one block per instance: inner convergence and beta
-__global__ void __launch_bounds__(RT) kb_final_update32(BatchArgs B) {
-    __shared__ double sh[2 * MAXQ][8];
-    const int slot = blockIdx.x;
-    if (slot >= B.n_inst) return;
+    __shared__ double sh[2][16];
+    __shared__ unsigned s_last;
+    const int slot = B.chunk2inst[blockIdx.x];
+    if (slot < 0) return;
     const BInst& I = B.inst[slot];
-    if (!I.active) return;
     BState* st = I.st;
-    if (st->odone || st->done) return;
-    double p[2];
-    inst_sums_plain<2>(p, B.pf + I.flat0, I.part.nflat, B.nflat, sh);
+    if (!I.active || st->odone || st->done) return;
+    const long long chunk = blockIdx.x - I.chunk0, Nn = I.part.Nn;
+    const int iter = st->iter;
+    const float alpha = (float)st->alpha;
+    const float* p = (iter & 1) ? I.p32b : I.p32a;
+    const bool fr = fi_now(st, FI_RV);
+    const long long fi_idx = fr ? st->fi_idx : -1;
+    double part[2] = {0.0, 0.0};
+    // four nodes from m on (the buffers are 256-byte aligned, m a multiple of 4); the end of the grid one by one
+    auto ld4 = [&](const float* v, long long m) {
+        if (m + 3 < Nn) return *reinterpret_cast<const float4*>(v + m);
+        return make_float4(m < Nn ? v[m] : 0.f, m + 1 < Nn ? v[m + 1] : 0.f, m + 2 < Nn ? v[m + 2] : 0.f, 0.f);
+    };
+    auto st4 = [&](float* v, long long m, float4 x) {
+        if (m + 3 < Nn) { *reinterpret_cast<float4*>(v + m) = x; return; }
+        if (m < Nn) v[m] = x.x;
+        if (m + 1 < Nn) v[m + 1] = x.y;
+        if (m + 2 < Nn) v[m + 2] = x.z;
+    };
+    float4 dv[UV], pv[UV], qv[UV], rv[UV], iv[UV];
+    const long long m0 = chunk * UC + threadIdx.x * 4;
+#pragma unroll
+    for (int u = 0; u < UV; ++u) {
+        const long long m = m0 + u * (RT * 4);
+        qv[u] = ld4(I.Ap32, m); rv[u] = ld4(I.r32, m); iv[u] = ld4(I.dinv32, m);
+        dv[u] = ld4(I.d32, m); pv[u] = ld4(p, m);
+    }
+#pragma unroll
+    for (int u = 0; u < UV; ++u) {
+        const long long m = m0 + u * (RT * 4);
+        float4 zv;
+        auto one = [&](int k, float& d, float pk, float q, float& r, float inv, float& z) {
+            d = __fmaf_rn(alpha, pk, d);
+            r = __fmaf_rn(-alpha, q, r);
+            if (fr && m + k == fi_idx) { r = flipf(r, st->fi_bit); st->fi_fired = 1; }
+            z = __fmul_rn(r, inv);
+            // products of FP32 values are exact in FP64; plain FP64 sums suffice
+            // for the inner solve's 1e-4 relative tolerance
+            part[0] = dfma((double)r, (double)r, part[0]);
+            part[1] = dfma((double)r, (double)z, part[1]);
+        };
+        one(0, dv[u].x, pv[u].x, qv[u].x, rv[u].x, iv[u].x, zv.x);
+        one(1, dv[u].y, pv[u].y, qv[u].y, rv[u].y, iv[u].y, zv.y);
+        one(2, dv[u].z, pv[u].z, qv[u].z, rv[u].z, iv[u].z, zv.z);
+        one(3, dv[u].w, pv[u].w, qv[u].w, rv[u].w, iv[u].w, zv.w);
+        st4(I.d32, m, dv[u]); st4(I.r32, m, rv[u]); st4(I.z32, m, zv);
+    }
+    if (!inst_finish<2, RT, 8>(part, B.pf + I.chunk0, B.nflat, chunk, I.nchunk, &st->tick_u, sh, &s_last)) return;
     if (threadIdx.x != 0) return;
     st->inner_total += 1;
-    const double rel = __ddiv_rn(__dsqrt_rn(p[0]), st->bn_in);
-    if (!isfinite(rel) || !isfinite(p[1])) { st->inner_bad = 1; st->done = 1; return; }
+    const double rel = __ddiv_rn(__dsqrt_rn(part[0]), st->bn_in);
+    if (!isfinite(rel) || !isfinite(part[1])) { st->inner_bad = 1; st->done = 1; return; }
     if (rel < st->tol_in || st->iter + 1 >= B.max_inner) { st->done = 1; return; }
-    st->beta = __ddiv_rn(p[1], st->rho);
-    st->rho = p[1];
+    st->beta = __ddiv_rn(part[1], st->rho);
+    st->rho = part[1];
     st->iter += 1;
 }
 
@@ -697,12 +903,13 @@ __global__ void k_recip32(long long n, const double* d, float* out) {
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
         out[i] = (float)__ddiv_rn(1.0, d[i]);
 }
-// interleaved FP64 and FP32 element coefficients (rho*c, k)
-__global__ void k_pack_coef(long long ne, const double* rhoc, const double* k, double2* c64, float2* c32) {
+// interleaved FP64 and FP32 element coefficients (rho*c, k); uniform rho*c: k alone in FP32
+__global__ void k_pack_coef(long long ne, const double* rhoc, const double* k, double2* c64, float2* c32, float* k32) {
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < ne; i += (long long)gridDim.x * blockDim.x) {
         const double r = rhoc[i], kk = k[i];
         c64[i] = make_double2(r, kk);
-        c32[i] = make_float2(__double2float_rn(r), __double2float_rn(kk));
+        if (k32) k32[i] = __double2float_rn(kk);
+        else c32[i] = make_float2(__double2float_rn(r), __double2float_rn(kk));
     }
 }
 // fresh state of an added instance: checksum weight norms from their squared sums, nothing to iterate
