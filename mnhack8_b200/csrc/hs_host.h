@@ -1,5 +1,6 @@
 // hs_host.h -- host-side set-up arithmetic shared by the library's translation units.
 #pragma once
+#include <cstddef>
 #include <cstdint>
 #include <string>
 #include <vector>
@@ -24,6 +25,12 @@ RefMatrices build_reference_matrices(int N);
 void build_source(int N, double src_sigma, std::vector<double>& F);
 void gaussian_ic(int N, double sigma, double* T);
 void exact_mode(int N, double t, double alpha, double* v);
+
+// Make the pages of a host buffer that a field is about to be copied into
+// resident (values unchanged), on several threads where that is worth it.  A
+// copy into fresh pages takes its page faults one by one inside the driver: a
+// 136 MB field 66 ms, 7 ms once the pages are there.
+void touch_pages(void* p, size_t bytes, bool parallel);
 
 void set_error(const std::string& msg);
 

@@ -1197,8 +1197,9 @@ __global__ void k_flip(double* v, long long idx, int bit) { v[idx] = flipbit(v[i
 struct StepCtl {
     int armR, vec, iter, bit;
     long long elem, idx;
-    int flipG, pad;
+    int flipG, max_iter;
     long long gidx;
+    double tol;
 };
 __global__ void k_step_begin(DevState* st, StepCtl c, double* T, unsigned* count) {
     st->stuck = 0;
@@ -1206,13 +1207,15 @@ __global__ void k_step_begin(DevState* st, StepCtl c, double* T, unsigned* count
     st->fi_armR = c.armR; st->fi_vec = c.vec; st->fi_iter = c.iter; st->fi_bit = c.bit;
     st->fi_elem = c.elem; st->fi_idx = c.idx;
     st->d1_step = 0.0;
+    st->max_iter = c.max_iter; st->tol = c.tol;
     if (c.flipG) T[c.gidx] = flipbit(T[c.gidx], c.bit);
 }
 __global__ void k_disarm_R(DevState* st) { st->fi_armR = 0; }
-__global__ void k_step_end(DevState* st, int* iters_out, double* d1_out) {
+__global__ void k_step_end(DevState* st, int* iters_out, double* d1_out, double* d1_last_out) {
     st->fi_armR = 0; st->fi_vec = 0;
     *iters_out = st->stuck ? -1 : st->result;
     *d1_out = st->d1_step;
+    if (d1_last_out) *d1_last_out = st->d1_last;
 }
 __global__ void k_d2_finish(const double* red, double* d2_out) {
     double bn = __dsqrt_rn(red[1]);

@@ -47,19 +47,37 @@ struct DevBuf {
     ~DevBuf() { if (p) cudaFree(p); }
 };
 
-// CUDA events released on every return path
+// Page-locked host memory that kernels write their results into, so that a call
+// ends with one synchronisation and no copy; kept by the handle and grown on demand
+template <class T>
+struct PinBuf {
+    T* p = nullptr;
+    size_t n = 0;
+    cudaError_t need(size_t count) {
+        if (count <= n) return cudaSuccess;
+        if (p) cudaFreeHost(p);
+        p = nullptr; n = 0;
+        const cudaError_t e = cudaMallocHost(&p, count * sizeof(T));
+        if (e == cudaSuccess) n = count;
+        return e;
+    }
+    ~PinBuf() { if (p) cudaFreeHost(p); }
+};
+
+// CUDA events, kept by the handle
 struct Events {
     std::vector<cudaEvent_t> e;
-    cudaError_t create(size_t n) {
-        e.assign(n, nullptr);
-        for (auto& v : e) {
+    cudaError_t need(size_t n) {
+        while (e.size() < n) {
+            cudaEvent_t v = nullptr;
             const cudaError_t r = cudaEventCreate(&v);
-            if (r != cudaSuccess) { v = nullptr; return r; }
+            if (r != cudaSuccess) return r;
+            e.push_back(v);
         }
         return cudaSuccess;
     }
     cudaEvent_t operator[](size_t i) const { return e[i]; }
-    ~Events() { for (auto v : e) if (v) cudaEventDestroy(v); }
+    ~Events() { for (auto v : e) cudaEventDestroy(v); }
 };
 
 inline int grid_for(long long n, int threads, int cap = 148 * 16) {
@@ -98,6 +116,13 @@ struct hs_solver {
     DevBuf<double> logs;                // diag-cg log buffers (3 * cap)
     DevBuf<double> T0;                  // initial condition kept on the device (hs_advance)
     bool has_F = false;
+    int max_iter = 0;                   // of the solves now launched (k_step_begin passes them on)
+    double tol = 0;
+
+    // results written by kernels (k_step_end and the detectors), and timing events
+    PinBuf<int> it_out;                 // per step: CG iterations (-1: a wait gave up)
+    PinBuf<double> rec_out;             // per step: d1, d2, tmin, tmax, E, spread, d1 of the last apply
+    Events ev;
 
     // PCG graphs built on first use: [0] step (RHS + PCG), [1] PCG only
     cudaGraph_t graph[2] = {nullptr, nullptr};
@@ -127,16 +152,18 @@ struct hs_solver {
 
 namespace {
 
-hs_status sync_state_config(hs_solver* h, int max_iter, double tol) {
-    DevState hs{};
-    std::memset(&hs, 0, sizeof(hs));
-    HS_CUDA(cudaMemcpyAsync(&hs, h->st.p, sizeof(DevState), cudaMemcpyDeviceToHost, h->s));
-    HS_CUDA(cudaStreamSynchronize(h->s));
-    hs.max_iter = max_iter;
-    hs.tol = tol;
-    HS_CUDA(cudaMemcpyAsync(h->st.p, &hs, sizeof(DevState), cudaMemcpyHostToDevice, h->s));
-    HS_CUDA(cudaStreamSynchronize(h->s));
+// room for the results of n steps
+hs_status need_out(hs_solver* h, int n) {
+    const size_t m = (size_t)std::max(n, 64);
+    HS_CUDA(h->it_out.need(m));
+    HS_CUDA(h->rec_out.need(m * 8));
     return HS_OK;
+}
+// the state at the start of a solve or a call: nothing armed, the handle's current limits
+StepCtl step_ctl(const hs_solver* h) {
+    StepCtl c{};
+    c.max_iter = h->max_iter; c.tol = h->tol;
+    return c;
 }
 
 int nblocks(const hs_solver* h) { return (int)h->part.nblk; }
@@ -452,7 +479,7 @@ hs_status build_graph(hs_solver* h, int which) {
 }
 
 hs_status arm_step(hs_solver* h, const hs_fi_spec* fi, int step, bool allow_G) {
-    StepCtl c{};
+    StepCtl c = step_ctl(h);
     if (fi && fi->level > 0 && fi->step == step) {
         if (fi->level == HS_FI_G) {
             if (allow_G) { c.flipG = 1; c.gidx = (long long)(fi->target % h->Nn); c.bit = fi->bit; }
@@ -669,7 +696,8 @@ hs_status hs_create(const hs_options* opt, const double* k_host, const double* r
     }
     HS_CUDA(cudaStreamSynchronize(h->s));
     HS_CUDA(cudaGetLastError());
-    hs_status st = sync_state_config(h.get(), opt->max_iter, opt->rtol);
+    h->max_iter = opt->max_iter; h->tol = opt->rtol;
+    const hs_status st = need_out(h.get(), 1);
     if (st != HS_OK) return st;
     *out = h.release();
     return HS_OK;
@@ -702,7 +730,7 @@ hs_status hs_apply(hs_solver* s, const double* x, double* y, double dt_eff, int 
         return HS_ERR_ARG;
     }
     if (abft_rel) *abft_rel = -1.0;
-    StepCtl c{};
+    StepCtl c = step_ctl(s);
     if (allow_fi && s->pending_set && s->pending.level == HS_FI_R) {
         c.armR = 1; c.elem = s->pending.target; c.bit = s->pending.bit;
         s->pending_set = false;
@@ -724,13 +752,12 @@ hs_status hs_apply(hs_solver* s, const double* x, double* y, double dt_eff, int 
         apply_projected(s, ROLE_RHS, x, y, dt_eff, d1, s->wM.p, nullptr, 0.0);
     else
         apply_projected(s, ROLE_X0, x, y, dt_eff, d1, s->wA.p, nullptr, 0.0);
-    k_step_end<<<1, 1, 0, s->s>>>(s->st.p, (int*)(s->red.p + 6), s->red.p + 7);
+    k_step_end<<<1, 1, 0, s->s>>>(s->st.p, s->it_out.p, s->rec_out.p, s->rec_out.p + 6);
     HS_CUDA(cudaGetLastError());
-    DevState hsx{};
-    HS_CUDA(cudaMemcpyAsync(&hsx, s->st.p, sizeof(hsx), cudaMemcpyDeviceToHost, s->s));
     HS_CUDA(cudaStreamSynchronize(s->s));
-    if (hsx.stuck) { const int bad = -1; return check_iters(&bad, 1); }
-    if (d1 && abft_rel) *abft_rel = hsx.d1_last;
+    const hs_status st = check_iters(s->it_out.p, 1);
+    if (st != HS_OK) return st;
+    if (d1 && abft_rel) *abft_rel = s->rec_out.p[6];
     return HS_OK;
 }
 
@@ -746,7 +773,7 @@ hs_status hs_build_rhs(hs_solver* s, const double* T, double* b) {
     if (!s || !T || !b) return HS_ERR_ARG;
     const bool src = !s->opt.verify && !s->opt.no_source && s->has_F;
     const bool d1 = s->opt.detect != 0;
-    k_step_begin<<<1, 1, 0, s->s>>>(s->st.p, StepCtl{}, s->T.p, s->ticket.p + 64);
+    k_step_begin<<<1, 1, 0, s->s>>>(s->st.p, step_ctl(s), s->T.p, s->ticket.p + 64);
     apply_projected(s, ROLE_RHS, T, b, 0.0, d1, s->wM.p, src ? s->F.p : nullptr, s->opt.dt);
     HS_CUDA(cudaGetLastError());
     HS_CUDA(cudaStreamSynchronize(s->s));
@@ -755,10 +782,10 @@ hs_status hs_build_rhs(hs_solver* s, const double* T, double* b) {
 
 hs_status hs_dot(hs_solver* s, const double* x, const double* y, double* out) {
     if (!s || !x || !y || !out) return HS_ERR_ARG;
-    launch_reduce(s, RED_DOT, x, y, s->red.p);
+    launch_reduce(s, RED_DOT, x, y, s->rec_out.p);
     HS_CUDA(cudaGetLastError());
-    HS_CUDA(cudaMemcpyAsync(out, s->red.p, 8, cudaMemcpyDeviceToHost, s->s));
     HS_CUDA(cudaStreamSynchronize(s->s));
+    *out = s->rec_out.p[0];
     return HS_OK;
 }
 
@@ -804,11 +831,29 @@ hs_status enqueue_step(hs_solver* h, const hs_fi_spec* fi, int step, int reproje
     }
     if (reproject) k_set_boundary<<<grid_for(h->Nn, RT), RT, 0, h->s>>>(h->N, h->T.p, 0.0);
     if (e1) HS_CUDA(cudaEventRecord(e1, h->s));
-    k_step_end<<<1, 1, 0, h->s>>>(h->st.p, d_iters, d_d1);
+    k_step_end<<<1, 1, 0, h->s>>>(h->st.p, d_iters, d_d1, nullptr);
     HS_CUDA(cudaGetLastError());
     return HS_OK;
 }
 
+}  // namespace
+
+namespace {
+// iteration limits of one call, in place of the handle's own
+struct Limits {
+    hs_solver* h;
+    Limits(hs_solver* h_, int max_iter, double tol) : h(h_) { h->max_iter = max_iter; h->tol = tol; }
+    ~Limits() { h->max_iter = h->opt.max_iter; h->tol = h->opt.rtol; }
+};
+// the initial condition on the device, kept by the handle
+hs_status need_T0(hs_solver* h) {
+    if (h->T0.p) return HS_OK;
+    std::vector<double> v(h->Nn, 0.0);
+    if (h->opt.ic_mode == 1) gaussian_ic(h->N, h->opt.ic_sigma, v.data());
+    HS_CUDA(h->T0.alloc(h->Nn));
+    HS_CUDA(cudaMemcpy(h->T0.p, v.data(), h->Nn * 8, cudaMemcpyHostToDevice));
+    return HS_OK;
+}
 }  // namespace
 
 // where a trajectory starts (run_case_impl)
@@ -825,10 +870,9 @@ extern "C" {
 
 hs_status hs_pcg(hs_solver* s, const double* b, double* x, int max_iter, double tol, int* iters) {
     if (!s || !b || !x) return HS_ERR_ARG;
-    hs_status st = sync_state_config(s, max_iter, tol);
+    hs_status st = build_graph(s, 1);
     if (st != HS_OK) return st;
-    st = build_graph(s, 1);
-    if (st != HS_OK) return st;
+    const Limits limits(s, max_iter, tol);
     HS_CUDA(cudaMemcpyAsync(s->b.p, b, s->Nn * 8, cudaMemcpyDeviceToDevice, s->s));
     HS_CUDA(cudaMemcpyAsync(s->T.p, x, s->Nn * 8, cudaMemcpyDeviceToDevice, s->s));
     hs_fi_spec fi{};
@@ -845,15 +889,14 @@ hs_status hs_pcg(hs_solver* s, const double* b, double* x, int max_iter, double 
         st = pcg_direct(s, false);
         if (st != HS_OK) return st;
     }
-    k_step_end<<<1, 1, 0, s->s>>>(s->st.p, (int*)(s->red.p + 6), s->red.p + 7);
+    k_step_end<<<1, 1, 0, s->s>>>(s->st.p, s->it_out.p, s->rec_out.p, nullptr);
     HS_CUDA(cudaGetLastError());
     HS_CUDA(cudaMemcpyAsync(x, s->T.p, s->Nn * 8, cudaMemcpyDeviceToDevice, s->s));
-    DevState hsx{};
-    HS_CUDA(cudaMemcpyAsync(&hsx, s->st.p, sizeof(hsx), cudaMemcpyDeviceToHost, s->s));
     HS_CUDA(cudaStreamSynchronize(s->s));
-    if (hsx.stuck) { const int bad = -1; return check_iters(&bad, 1); }
-    if (iters) *iters = hsx.result;
-    return sync_state_config(s, s->opt.max_iter, s->opt.rtol);
+    st = check_iters(s->it_out.p, 1);
+    if (st != HS_OK) return st;
+    if (iters) *iters = s->it_out.p[0];
+    return HS_OK;
 }
 
 hs_status hs_run_case(hs_solver* h, int n_steps, int snap_every, const hs_fi_spec* fi, int reproject,
@@ -878,8 +921,6 @@ hs_status run_case_impl(hs_solver* h, int n_steps, int snap_every, const hs_fi_s
     }
     hs_status st = validate_fi(h, fi);
     if (st != HS_OK) return st;
-    st = sync_state_config(h, h->opt.max_iter, h->opt.rtol);
-    if (st != HS_OK) return st;
     st = build_graph(h, 0);
     if (st != HS_OK) return st;
     const long long Nn = h->Nn;
@@ -888,10 +929,9 @@ hs_status run_case_impl(hs_solver* h, int n_steps, int snap_every, const hs_fi_s
     if (s0 > 0) {
         HS_CUDA(cudaMemcpyAsync(h->T.p, from.T_start, Nn * 8, cudaMemcpyDeviceToDevice, h->s));
     } else if (h->opt.ic_mode == 1) {
-        std::vector<double> T0(Nn);
-        gaussian_ic(h->N, h->opt.ic_sigma, T0.data());
-        HS_CUDA(cudaMemcpyAsync(h->T.p, T0.data(), Nn * 8, cudaMemcpyHostToDevice, h->s));
-        HS_CUDA(cudaStreamSynchronize(h->s));
+        st = need_T0(h);
+        if (st != HS_OK) return st;
+        HS_CUDA(cudaMemcpyAsync(h->T.p, h->T0.p, Nn * 8, cudaMemcpyDeviceToDevice, h->s));
     } else {
         HS_CUDA(cudaMemsetAsync(h->T.p, 0, Nn * 8, h->s));
     }
@@ -910,22 +950,20 @@ hs_status run_case_impl(hs_solver* h, int n_steps, int snap_every, const hs_fi_s
         }
         h->ref_nsteps = n_steps; h->ref_snap_every = snap_every;
     }
-    // per-step device outputs
-    DevBuf<int> d_it;
-    DevBuf<double> d_rec;   // per step: d1, d2, tmin, tmax, E, spread
-    HS_CUDA(d_it.alloc(std::max(n_steps, 1)));
-    HS_CUDA(d_rec.alloc((size_t)std::max(n_steps, 1) * 8));
-    HS_CUDA(cudaMemsetAsync(d_rec.p, 0, (size_t)std::max(n_steps, 1) * 8 * 8, h->s));
-    Events ev;
-    HS_CUDA(ev.create(2 * (size_t)n_steps));
+    // per-step outputs: d1, d2, tmin, tmax, E, spread
+    st = need_out(h, n_steps);
+    if (st != HS_OK) return st;
+    std::fill(h->rec_out.p, h->rec_out.p + (size_t)n_steps * 8, 0.0);
+    Events& ev = h->ev;
+    HS_CUDA(ev.need(2 * (size_t)n_steps));
     int si = 0;
     for (int step = 0; step < s0; ++step)
         if ((snap_every > 0 && step % snap_every == 0) || step == n_steps - 1) ++si;
     for (int step = s0; step < n_steps; ++step) {
-        double* rec = d_rec.p + (size_t)step * 8;
+        double* rec = h->rec_out.p + (size_t)step * 8;
         if (from.keep_states)
             HS_CUDA(cudaMemcpyAsync(from.keep_states[step], h->T.p, Nn * 8, cudaMemcpyDeviceToDevice, h->s));
-        st = enqueue_step(h, fi, step, reproject, d_it.p + step, rec + 0, ev[2 * step], ev[2 * step + 1]);
+        st = enqueue_step(h, fi, step, reproject, h->it_out.p + step, rec + 0, ev[2 * step], ev[2 * step + 1]);
         if (st != HS_OK) return st;
         if (h->opt.detect) {
             // D2: true residual with a fresh matvec (het.cu:1205-1210); D3 range (het.cu:1219)
@@ -962,12 +1000,11 @@ hs_status run_case_impl(hs_solver* h, int n_steps, int snap_every, const hs_fi_s
         }
         HS_CUDA(cudaGetLastError());
     }
+    if (T_final_host) touch_pages(T_final_host, Nn * 8, false);        // while the device works
     HS_CUDA(cudaStreamSynchronize(h->s));
-    std::vector<int> it(std::max(n_steps, 1));
-    std::vector<double> rec((size_t)std::max(n_steps, 1) * 8);
-    HS_CUDA(cudaMemcpy(it.data(), d_it.p, n_steps * sizeof(int), cudaMemcpyDeviceToHost));
-    HS_CUDA(cudaMemcpy(rec.data(), d_rec.p, (size_t)n_steps * 8 * 8, cudaMemcpyDeviceToHost));
-    st = check_iters(it.data() + s0, n_steps - s0);
+    const int* it = h->it_out.p;
+    const double* rec = h->rec_out.p;
+    st = check_iters(it + s0, n_steps - s0);
     if (st != HS_OK) return st;
     int nf = 0;
     si = 0;
@@ -1006,34 +1043,28 @@ hs_status hs_verify(hs_solver* h, int n_steps, double* rel_err, long long* total
         set_error(msg);
         return HS_ERR_ARG;
     }
-    hs_status st = sync_state_config(h, h->opt.max_iter, h->opt.rtol);
-    if (st != HS_OK) return st;
-    st = build_graph(h, 0);
+    hs_status st = build_graph(h, 0);
     if (st != HS_OK) return st;
     const double alpha = h->kmin / h->rhocmin;
     const long long Nn = h->Nn;
     std::vector<double> v(Nn);
     exact_mode(h->N, 0.0, alpha, v.data());
     HS_CUDA(cudaMemcpyAsync(h->T.p, v.data(), Nn * 8, cudaMemcpyHostToDevice, h->s));
-    DevBuf<int> d_it;
-    DevBuf<double> d_d1;
-    HS_CUDA(d_it.alloc(std::max(n_steps, 1)));
-    HS_CUDA(d_d1.alloc(std::max(n_steps, 1)));
-    Events ev2;
-    HS_CUDA(ev2.create(2));
-    cudaEvent_t e0 = ev2[0], e1 = ev2[1];
+    st = need_out(h, n_steps);
+    if (st != HS_OK) return st;
+    HS_CUDA(h->ev.need(2));
+    cudaEvent_t e0 = h->ev[0], e1 = h->ev[1];
     HS_CUDA(cudaEventRecord(e0, h->s));
     for (int step = 0; step < n_steps; ++step) {
-        st = enqueue_step(h, nullptr, step, 0, d_it.p + step, d_d1.p + step, nullptr, nullptr);
+        st = enqueue_step(h, nullptr, step, 0, h->it_out.p + step, h->rec_out.p + step, nullptr, nullptr);
         if (st != HS_OK) return st;
     }
     HS_CUDA(cudaEventRecord(e1, h->s));
     HS_CUDA(cudaEventSynchronize(e1));
     float fms = 0.f;
     HS_CUDA(cudaEventElapsedTime(&fms, e0, e1));
-    std::vector<int> it(std::max(n_steps, 1));
-    HS_CUDA(cudaMemcpy(it.data(), d_it.p, n_steps * sizeof(int), cudaMemcpyDeviceToHost));
-    st = check_iters(it.data(), n_steps);
+    const int* it = h->it_out.p;
+    st = check_iters(it, n_steps);
     if (st != HS_OK) return st;
     long long tot = 0;
     for (int i = 0; i < n_steps; ++i) tot += it[i];
@@ -1058,27 +1089,24 @@ hs_status hs_solve_host(hs_solver* h, const double* T0_host, double* T_host, int
     hs_status st = build_graph(h, 0);
     if (st != HS_OK) return st;
     const long long Nn = h->Nn;
-    DevBuf<int> d_it;
-    DevBuf<double> d_d1;
-    HS_CUDA(d_it.alloc(std::max(n_steps, 1)));
-    HS_CUDA(d_d1.alloc(std::max(n_steps, 1)));
-    Events ev2;
-    HS_CUDA(ev2.create(2));
-    cudaEvent_t e0 = ev2[0], e1 = ev2[1];
+    st = need_out(h, n_steps);
+    if (st != HS_OK) return st;
+    HS_CUDA(h->ev.need(2));
+    cudaEvent_t e0 = h->ev[0], e1 = h->ev[1];
     HS_CUDA(cudaEventRecord(e0, h->s));
     HS_CUDA(cudaMemcpyAsync(h->T.p, T0_host, Nn * 8, cudaMemcpyHostToDevice, h->s));
     for (int step = 0; step < n_steps; ++step) {
-        st = enqueue_step(h, nullptr, step, 0, d_it.p + step, d_d1.p + step, nullptr, nullptr);
+        st = enqueue_step(h, nullptr, step, 0, h->it_out.p + step, h->rec_out.p + step, nullptr, nullptr);
         if (st != HS_OK) return st;
     }
+    touch_pages(T_host, Nn * 8, false);        // while the device works
     HS_CUDA(cudaMemcpyAsync(T_host, h->T.p, Nn * 8, cudaMemcpyDeviceToHost, h->s));
     HS_CUDA(cudaEventRecord(e1, h->s));
     HS_CUDA(cudaEventSynchronize(e1));
     float fms = 0.f;
     HS_CUDA(cudaEventElapsedTime(&fms, e0, e1));
-    std::vector<int> it(std::max(n_steps, 1));
-    HS_CUDA(cudaMemcpy(it.data(), d_it.p, n_steps * sizeof(int), cudaMemcpyDeviceToHost));
-    st = check_iters(it.data(), n_steps);
+    const int* it = h->it_out.p;
+    st = check_iters(it, n_steps);
     if (st != HS_OK) return st;
     long long tot = 0;
     for (int i = 0; i < n_steps; ++i) tot += it[i];
@@ -1121,8 +1149,7 @@ int hs_target_on_boundary(const hs_solver* s, const hs_fi_spec* fi) {
 hs_status hs_diag_cg(hs_solver* h, int max_iter, double tol, double* rel0, double* rel, double* alpha, double* beta,
                      int cap, int* iters) {
     if (!h || cap < 0) return HS_ERR_ARG;
-    hs_status st = sync_state_config(h, max_iter, tol);
-    if (st != HS_OK) return st;
+    const Limits limits(h, max_iter, tol);
     DevBuf<double> lg;
     HS_CUDA(lg.alloc((size_t)3 * std::max(cap, 1)));
     DevState hsx{};
@@ -1133,16 +1160,12 @@ hs_status hs_diag_cg(hs_solver* h, int max_iter, double tol, double* rel0, doubl
     std::vector<double> T0(h->Nn, 0.0);
     if (h->opt.ic_mode == 1) gaussian_ic(h->N, h->opt.ic_sigma, T0.data());
     HS_CUDA(cudaMemcpyAsync(h->T.p, T0.data(), h->Nn * 8, cudaMemcpyHostToDevice, h->s));
-    st = build_graph(h, 0);
+    hs_status st = build_graph(h, 0);
     if (st != HS_OK) return st;
-    DevBuf<int> d_it;
-    DevBuf<double> d_d1;
-    HS_CUDA(d_it.alloc(1)); HS_CUDA(d_d1.alloc(1));
-    st = enqueue_step(h, nullptr, 0, 0, d_it.p, d_d1.p, nullptr, nullptr);
+    st = enqueue_step(h, nullptr, 0, 0, h->it_out.p, h->rec_out.p, nullptr, nullptr);
     if (st != HS_OK) return st;
     HS_CUDA(cudaStreamSynchronize(h->s));
-    int it = 0;
-    HS_CUDA(cudaMemcpy(&it, d_it.p, sizeof(int), cudaMemcpyDeviceToHost));
+    const int it = h->it_out.p[0];
     st = check_iters(&it, 1);
     if (st != HS_OK) return st;
     HS_CUDA(cudaMemcpy(&hsx, h->st.p, sizeof(hsx), cudaMemcpyDeviceToHost));
@@ -1154,7 +1177,7 @@ hs_status hs_diag_cg(hs_solver* h, int max_iter, double tol, double* rel0, doubl
     if (iters) *iters = it;
     hsx.log_rel = hsx.log_alpha = hsx.log_beta = nullptr; hsx.log_cap = 0;
     HS_CUDA(cudaMemcpy(h->st.p, &hsx, sizeof(hsx), cudaMemcpyHostToDevice));
-    return sync_state_config(h, h->opt.max_iter, h->opt.rtol);
+    return HS_OK;
 }
 
 }  // extern "C"
@@ -1170,6 +1193,7 @@ hs_status hs_set_field(hs_solver* h, const double* T_host) {
 
 hs_status hs_get_field(hs_solver* h, double* T_host) {
     if (!h || !T_host) return HS_ERR_ARG;
+    touch_pages(T_host, h->Nn * 8, true);
     HS_CUDA(cudaMemcpyAsync(T_host, h->T.p, h->Nn * 8, cudaMemcpyDeviceToHost, h->s));
     HS_CUDA(cudaStreamSynchronize(h->s));
     return HS_OK;
@@ -1179,32 +1203,26 @@ hs_status hs_advance(hs_solver* h, int n_steps, int from_ic, long long* total_it
     if (!h || n_steps < 0) return HS_ERR_ARG;
     hs_status st = build_graph(h, 0);
     if (st != HS_OK) return st;
-    if (from_ic && !h->T0.p) {
-        std::vector<double> v(h->Nn, 0.0);
-        if (h->opt.ic_mode == 1) gaussian_ic(h->N, h->opt.ic_sigma, v.data());
-        HS_CUDA(h->T0.alloc(h->Nn));
-        HS_CUDA(cudaMemcpy(h->T0.p, v.data(), h->Nn * 8, cudaMemcpyHostToDevice));
+    if (from_ic) {
+        st = need_T0(h);
+        if (st != HS_OK) return st;
     }
-    DevBuf<int> d_it;
-    DevBuf<double> d_d1;
-    HS_CUDA(d_it.alloc(std::max(n_steps, 1)));
-    HS_CUDA(d_d1.alloc(std::max(n_steps, 1)));
-    Events ev2;
-    HS_CUDA(ev2.create(2));
-    cudaEvent_t e0 = ev2[0], e1 = ev2[1];
+    st = need_out(h, n_steps);
+    if (st != HS_OK) return st;
+    HS_CUDA(h->ev.need(2));
+    cudaEvent_t e0 = h->ev[0], e1 = h->ev[1];
     HS_CUDA(cudaEventRecord(e0, h->s));
     if (from_ic) HS_CUDA(cudaMemcpyAsync(h->T.p, h->T0.p, h->Nn * 8, cudaMemcpyDeviceToDevice, h->s));
     for (int step = 0; step < n_steps; ++step) {
-        st = enqueue_step(h, nullptr, step, 0, d_it.p + step, d_d1.p + step, nullptr, nullptr);
+        st = enqueue_step(h, nullptr, step, 0, h->it_out.p + step, h->rec_out.p + step, nullptr, nullptr);
         if (st != HS_OK) return st;
     }
     HS_CUDA(cudaEventRecord(e1, h->s));
     HS_CUDA(cudaEventSynchronize(e1));
     float fms = 0.f;
     HS_CUDA(cudaEventElapsedTime(&fms, e0, e1));
-    std::vector<int> it(std::max(n_steps, 1));
-    HS_CUDA(cudaMemcpy(it.data(), d_it.p, n_steps * sizeof(int), cudaMemcpyDeviceToHost));
-    st = check_iters(it.data(), n_steps);
+    const int* it = h->it_out.p;
+    st = check_iters(it, n_steps);
     if (st != HS_OK) return st;
     long long tot = 0;
     for (int i = 0; i < n_steps; ++i) tot += it[i];
@@ -1231,8 +1249,8 @@ hs_status hs_time_kernel(hs_solver* h, int which, int reps, double* ms_per_launc
     const size_t fl = (size_t)32 << 20;   // doubles
     HS_CUDA(flush.alloc(fl));
     HS_CUDA(cudaMemsetAsync(flush.p, 0, fl * 8, h->s));
-    Events ev;
-    HS_CUDA(ev.create(2 * (size_t)reps));
+    Events& ev = h->ev;
+    HS_CUDA(ev.need(2 * (size_t)reps));
     const bool det = h->opt.detect != 0;
     // the update finishes the operator's reductions: give it one operator's partials
     if (which == 1) apply_projected(h, ROLE_LOOP, nullptr, h->Ap.p, h->opt.dt, det, h->wA.p, nullptr, 0.0);
