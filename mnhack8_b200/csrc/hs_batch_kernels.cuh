@@ -83,7 +83,9 @@ struct BState {
     int has_prev;           // the previous step's field is kept (extrapolated start)
     int extrap;             // this step starts from 2 T - T_prev
     unsigned tick_a, tick_u;   // blocks of the running inner apply / update that are done
-    int stuck, pad3;        // a bounded wait gave up: the inner solve is discarded
+    int stuck;              // a bounded wait gave up: the inner solve is discarded
+    int pend;               // d += alpha p of the last (even) inner iteration is still owed
+    double alpha_prev;      // alpha of the inner iteration before
 };
 
 __device__ __forceinline__ float flipf(float x, int bit) {
@@ -668,7 +670,7 @@ __global__ void __launch_bounds__(FT, 2) kb_apply32(BatchArgs B) {
     st->applies32 += 1;
     if (!isfinite(part[0]) || st->stuck) { st->inner_bad = 1; st->done = 1; st->stuck = 0; }
     else if (fabs(part[0]) < 1e-30) { st->broken = 1; st->done = 1; }
-    else st->alpha = __ddiv_rn(st->rho, part[0]);
+    else { st->alpha_prev = st->alpha; st->alpha = __ddiv_rn(st->rho, part[0]); }
 }
 
 // compensated sums of one instance's partials: count (hi, lo) pairs per
@@ -798,18 +800,24 @@ __global__ void __launch_bounds__(RT) kb_outer_final(BatchArgs B) {
     st->bn_in = __dsqrt_rn(p[3]);
     // solve only as far as the outer target needs: max(inner_tol, rtol / (2 rel64))
     st->tol_in = fmax(B.inner_tol, __ddiv_rn(0.5 * B.rtol, st->rel64));
-    st->iter = 0; st->broken = 0; st->beta = 0.0; st->inner_bad = 0;
+    st->iter = 0; st->broken = 0; st->beta = 0.0; st->inner_bad = 0; st->pend = 0;
     st->done = (st->bn_in < 1e-300 || !isfinite(st->bn_in) || !isfinite(p[2])) ? 1 : 0;
     if (!isfinite(st->bn_in) || !isfinite(p[2])) st->inner_bad = 1;
 }
 
 // ---- the FP32 inner loop: vector update ----------------------------------------------
-// d += alpha p, r -= alpha Ap, z = r / diag; r.r and r.z.  A block takes a chunk
-// of UC consecutive nodes, UV groups of four per thread with every load in
-// flight at once; the last block of an instance to finish adds up its chunks'
-// sums and does the inner solve's scalar step (beta, convergence).
-constexpr int UV = 2, UC = RT * 4 * UV;
-__global__ void __launch_bounds__(RT) kb_update32(BatchArgs B) {
+// r -= alpha Ap, z = r / diag; r.r and r.z; and at odd iterations d += alpha p
+// for the previous iteration and this one (the same two multiply-adds in the
+// same order; the previous p is still in the other buffer), which saves 4 of 32
+// bytes per node on average.  A block takes a chunk of UC consecutive nodes in
+// UL rounds of UV groups of four per thread, a round's loads in flight together;
+// the last block of an instance to finish adds up its chunks' sums and does the
+// inner solve's scalar step (beta, convergence).  The block's tree, fence and
+// ticket are what a chunk must outweigh (24 instances of N 16..96 / N=160, device
+// ms: 1024 nodes 170 / 175, 2048 148 / 148; with d every second iteration at 64
+// registers 2048 150 / 150, 4096 147 / 148, 8192 145 / 145).
+constexpr int UV = 2, UL = 4, UC = RT * 4 * UV * UL;
+__global__ void __launch_bounds__(RT, 4) kb_update32(BatchArgs B) {
     __shared__ double sh[2][16];
     __shared__ unsigned s_last;
     const int slot = B.chunk2inst[blockIdx.x];
@@ -820,7 +828,8 @@ __global__ void __launch_bounds__(RT) kb_update32(BatchArgs B) {
     const long long chunk = blockIdx.x - I.chunk0, Nn = I.part.Nn;
     const int iter = st->iter;
     const float alpha = (float)st->alpha;
-    const float* p = (iter & 1) ? I.p32b : I.p32a;
+    const bool odd = iter & 1;
+    const float alpha_prev = odd ? (float)st->alpha_prev : 0.f;
     const bool fr = fi_now(st, FI_RV);
     const long long fi_idx = fr ? st->fi_idx : -1;
     double part[2] = {0.0, 0.0};
@@ -835,37 +844,45 @@ __global__ void __launch_bounds__(RT) kb_update32(BatchArgs B) {
         if (m + 1 < Nn) v[m + 1] = x.y;
         if (m + 2 < Nn) v[m + 2] = x.z;
     };
-    float4 dv[UV], pv[UV], qv[UV], rv[UV], iv[UV];
-    const long long m0 = chunk * UC + threadIdx.x * 4;
+    float4 dv[UV], pv[UV], ov[UV], qv[UV], rv[UV], iv[UV];
+    for (int ul = 0; ul < UL; ++ul) {
+        const long long m0 = chunk * UC + ul * (RT * 4 * UV) + threadIdx.x * 4;
 #pragma unroll
-    for (int u = 0; u < UV; ++u) {
-        const long long m = m0 + u * (RT * 4);
-        qv[u] = ld4(I.Ap32, m); rv[u] = ld4(I.r32, m); iv[u] = ld4(I.dinv32, m);
-        dv[u] = ld4(I.d32, m); pv[u] = ld4(p, m);
-    }
+        for (int u = 0; u < UV; ++u) {
+            const long long m = m0 + u * (RT * 4);
+            qv[u] = ld4(I.Ap32, m); rv[u] = ld4(I.r32, m); iv[u] = ld4(I.dinv32, m);
+            if (odd) { dv[u] = ld4(I.d32, m); pv[u] = ld4(I.p32b, m); ov[u] = ld4(I.p32a, m); }
+        }
 #pragma unroll
-    for (int u = 0; u < UV; ++u) {
-        const long long m = m0 + u * (RT * 4);
-        float4 zv;
-        auto one = [&](int k, float& d, float pk, float q, float& r, float inv, float& z) {
-            d = __fmaf_rn(alpha, pk, d);
-            r = __fmaf_rn(-alpha, q, r);
-            if (fr && m + k == fi_idx) { r = flipf(r, st->fi_bit); st->fi_fired = 1; }
-            z = __fmul_rn(r, inv);
-            // products of FP32 values are exact in FP64; plain FP64 sums suffice
-            // for the inner solve's 1e-4 relative tolerance
-            part[0] = dfma((double)r, (double)r, part[0]);
-            part[1] = dfma((double)r, (double)z, part[1]);
-        };
-        one(0, dv[u].x, pv[u].x, qv[u].x, rv[u].x, iv[u].x, zv.x);
-        one(1, dv[u].y, pv[u].y, qv[u].y, rv[u].y, iv[u].y, zv.y);
-        one(2, dv[u].z, pv[u].z, qv[u].z, rv[u].z, iv[u].z, zv.z);
-        one(3, dv[u].w, pv[u].w, qv[u].w, rv[u].w, iv[u].w, zv.w);
-        st4(I.d32, m, dv[u]); st4(I.r32, m, rv[u]); st4(I.z32, m, zv);
+        for (int u = 0; u < UV; ++u) {
+            const long long m = m0 + u * (RT * 4);
+            float4 zv;
+            if (odd) {
+                auto add = [&](float& d, float po, float pk) { d = __fmaf_rn(alpha, pk, __fmaf_rn(alpha_prev, po, d)); };
+                add(dv[u].x, ov[u].x, pv[u].x); add(dv[u].y, ov[u].y, pv[u].y);
+                add(dv[u].z, ov[u].z, pv[u].z); add(dv[u].w, ov[u].w, pv[u].w);
+                st4(I.d32, m, dv[u]);
+            }
+            auto one = [&](int k, float q, float& r, float inv, float& z) {
+                r = __fmaf_rn(-alpha, q, r);
+                if (fr && m + k == fi_idx) { r = flipf(r, st->fi_bit); st->fi_fired = 1; }
+                z = __fmul_rn(r, inv);
+                // products of FP32 values are exact in FP64; plain FP64 sums suffice
+                // for the inner solve's 1e-4 relative tolerance
+                part[0] = dfma((double)r, (double)r, part[0]);
+                part[1] = dfma((double)r, (double)z, part[1]);
+            };
+            one(0, qv[u].x, rv[u].x, iv[u].x, zv.x);
+            one(1, qv[u].y, rv[u].y, iv[u].y, zv.y);
+            one(2, qv[u].z, rv[u].z, iv[u].z, zv.z);
+            one(3, qv[u].w, rv[u].w, iv[u].w, zv.w);
+            st4(I.r32, m, rv[u]); st4(I.z32, m, zv);
+        }
     }
     if (!inst_finish<2, RT, 8>(part, B.pf + I.chunk0, B.nflat, chunk, I.nchunk, &st->tick_u, sh, &s_last)) return;
     if (threadIdx.x != 0) return;
     st->inner_total += 1;
+    st->pend = odd ? 0 : 1;
     const double rel = __ddiv_rn(__dsqrt_rn(part[0]), st->bn_in);
     if (!isfinite(rel) || !isfinite(part[1])) { st->inner_bad = 1; st->done = 1; return; }
     if (rel < st->tol_in || st->iter + 1 >= B.max_inner) { st->done = 1; return; }
@@ -883,9 +900,14 @@ __global__ void __launch_bounds__(RT) kb_correct(BatchArgs B) {
     const BInst& I = B.inst[f.slot];
     if (!I.active || I.st->odone || I.st->inner_bad) return;
     const int N = I.part.N;
+    // an even last iteration's p is in p32a (a later p, if any, went to p32b)
+    const bool pend = I.st->pend != 0;
+    const float alpha = (float)I.st->alpha;
     for (int k = 0; k < f.cnt; ++k) {
         const long long m = f.m0 + k;
-        if (!is_bnd(m, N)) I.T[m] = dadd(I.T[m], (double)I.d32[m]);
+        if (is_bnd(m, N)) continue;
+        const float d = pend ? __fmaf_rn(alpha, I.p32a[m], I.d32[m]) : I.d32[m];
+        I.T[m] = dadd(I.T[m], (double)d);
     }
 }
 

@@ -1,5 +1,5 @@
 """The batched engine's FP32 inner loop at the sizes where it can go wrong:
-grids whose nodes are not a multiple of four or of the update's chunk of 2048
+grids whose nodes are not a multiple of four or of the update's chunk of 8192
 nodes (1, 2, 12, 13), tiles with one and with several rows of positions per
 thread (13, 29, 40), several tiles per plane (40), uniform rho*c (read as one
 value) and varying rho*c, checksum on and off.
