@@ -111,6 +111,12 @@ def reduce_over_ranks(dist, elapsed, iters, device):
     return float(t[0]), float(t[1])
 
 
+def coef_bytes(kernel, scatter, rhoc):
+    """Coefficient bytes the operator reads per element: (rho*c, k), or k alone
+    where the wht form finds rho*c to be one value."""
+    return 8 if kernel == "wht" and scatter == "colored" and float(np.min(rhoc)) == float(np.max(rhoc)) else 16
+
+
 def peaks():
     p = os.path.join(ROOT, "MEASURED_PEAKS.json")
     if os.path.exists(p):
@@ -392,7 +398,8 @@ def main():
     ms_k1 = g.time_kernel(0, reps=20)
     ms_k2 = g.time_kernel(1, reps=20)
     detect = not args.no_detect
-    alg_k1 = (40 if detect else 32) * nodes + 16 * elems   # read z, p_old[, w]; write p, Ap; read k, rho*c
+    # read z, p_old[, w]; write p, Ap; read k[, rho*c]
+    alg_k1 = (40 if detect else 32) * nodes + coef_bytes(args.kernel, args.scatter, r) * elems
     # the update at an odd iteration (timed): read x, p_{k-1}, p_k, Ap, r, d; write x, r, z
     # (an even iteration skips x: read Ap, r, d; write r, z)
     alg_k2 = 72 * nodes
@@ -467,7 +474,7 @@ def profile_kernel(args):
                     no_source=True, ic="gaussian", ic_sigma=IC_SIGMA, rtol=RTOL, max_iter=500, device=0)
     ms = g.time_kernel(0, reps=PROFILE_REPS)
     g.close()
-    alg = (40 if not args.no_detect else 32) * (N + 1) ** 3 + 16 * N ** 3
+    alg = (40 if not args.no_detect else 32) * (N + 1) ** 3 + coef_bytes(args.kernel, args.scatter, r) * N ** 3
     print(json.dumps({"N": N, "ms_per_launch": ms, "alg_bytes_per_launch": alg,
                       "achieved_gbs": alg / (ms * 1e-3) / 1e9}), flush=True)
     return 0
@@ -515,7 +522,7 @@ def gate_apply(device, detect, kernel, scatter):
     g.time_kernel(0, reps=3)
     ms = min(g.time_kernel(0, reps=20) for _ in range(2))
     g.close()
-    alg = (40 if detect else 32) * nodes + 16 * elems
+    alg = (40 if detect else 32) * nodes + coef_bytes(kernel, scatter, r) * elems
     peak, kind = peaks()
     ach = alg / (ms * 1e-3) / 1e9
     return {"N": N, "ms_per_launch": ms, "alg_bytes_per_launch": alg, "achieved": ach, "peak": peak,

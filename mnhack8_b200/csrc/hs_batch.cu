@@ -628,7 +628,7 @@ hs_status hs_batch_get_field(hs_batch* b, int slot, double* T_host) {
     }
     HS_CUDA(cudaSetDevice(b->opt.device));
     const auto& sl = b->slots[slot];
-    touch_pages(T_host, sl.part.Nn * 8, true);
+    touch_output(T_host, sl.part.Nn * 8, true);
     HS_CUDA(cudaMemcpyAsync(T_host, sl.desc.T, sl.part.Nn * 8, cudaMemcpyDeviceToHost, b->s));
     HS_CUDA(cudaStreamSynchronize(b->s));
     return HS_OK;

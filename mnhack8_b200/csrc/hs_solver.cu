@@ -80,6 +80,14 @@ struct Events {
     ~Events() { for (auto v : e) cudaEventDestroy(v); }
 };
 
+// touch_pages for a caller's output buffer; a device address is left to the
+// copy, which refuses it
+void touch_output(void* p, size_t bytes, bool parallel) {
+    cudaPointerAttributes at{};
+    if (cudaPointerGetAttributes(&at, p) != cudaSuccess) { cudaGetLastError(); return; }
+    if (at.type != cudaMemoryTypeDevice) touch_pages(p, bytes, parallel);
+}
+
 inline int grid_for(long long n, int threads, int cap = 148 * 16) {
     long long g = (n + threads - 1) / threads;
     if (g > cap) g = cap;
@@ -1000,7 +1008,7 @@ hs_status run_case_impl(hs_solver* h, int n_steps, int snap_every, const hs_fi_s
         }
         HS_CUDA(cudaGetLastError());
     }
-    if (T_final_host) touch_pages(T_final_host, Nn * 8, false);        // while the device works
+    if (T_final_host) touch_output(T_final_host, Nn * 8, false);        // while the device works
     HS_CUDA(cudaStreamSynchronize(h->s));
     const int* it = h->it_out.p;
     const double* rec = h->rec_out.p;
@@ -1099,7 +1107,7 @@ hs_status hs_solve_host(hs_solver* h, const double* T0_host, double* T_host, int
         st = enqueue_step(h, nullptr, step, 0, h->it_out.p + step, h->rec_out.p + step, nullptr, nullptr);
         if (st != HS_OK) return st;
     }
-    touch_pages(T_host, Nn * 8, false);        // while the device works
+    touch_output(T_host, Nn * 8, false);        // while the device works
     HS_CUDA(cudaMemcpyAsync(T_host, h->T.p, Nn * 8, cudaMemcpyDeviceToHost, h->s));
     HS_CUDA(cudaEventRecord(e1, h->s));
     HS_CUDA(cudaEventSynchronize(e1));
@@ -1193,7 +1201,7 @@ hs_status hs_set_field(hs_solver* h, const double* T_host) {
 
 hs_status hs_get_field(hs_solver* h, double* T_host) {
     if (!h || !T_host) return HS_ERR_ARG;
-    touch_pages(T_host, h->Nn * 8, true);
+    touch_output(T_host, h->Nn * 8, true);
     HS_CUDA(cudaMemcpyAsync(T_host, h->T.p, h->Nn * 8, cudaMemcpyDeviceToHost, h->s));
     HS_CUDA(cudaStreamSynchronize(h->s));
     return HS_OK;
