@@ -64,3 +64,36 @@ def test_iteration_cap_and_zero_rhs(oracle, N, cap):
     it_ref, x_ref, _ = o.pcg(z, z, cap, 1e-12)
     assert it == it_ref and np.array_equal(bits(dev.get(xd)), bits(x_ref))
     g.close()
+
+
+def test_handles_in_threads(oracle):
+    """Cooperative solves of several handles from several threads, beside a
+    batched engine's steps: each gives the bits it gives alone."""
+    import threading
+
+    probs = [(48, "wht"), (30, "fast"), (60, "wht")]
+    solvers = [pair(oracle, N, form)[1] for N, form in probs]
+
+    def solve(i, out):
+        for _ in range(3):
+            solvers[i].advance(4, from_ic=True)
+        out[i] = solvers[i].get_field()
+
+    alone, mixed = {}, {}
+    for i in range(len(probs)):
+        solve(i, alone)
+    k, r = field(40, "lognormal", sigma=1.0, L=0.25, seed=3)
+    b = _lib.Batch(rtol=1e-8)
+    s = [b.add(40, 5e-4, k, r, T0=_lib.gaussian_ic(40, 0.15), steps=20) for _ in range(2)]
+    th = [threading.Thread(target=solve, args=(i, mixed)) for i in range(len(probs))]
+    for t in th:
+        t.start()
+    while b.step()[0]:
+        pass
+    for t in th:
+        t.join()
+    for i in range(len(probs)):
+        assert np.array_equal(bits(alone[i]), bits(mixed[i])), probs[i]
+        solvers[i].close()
+    assert np.array_equal(bits(b.field(s[0])), bits(b.field(s[1])))
+    b.close()
