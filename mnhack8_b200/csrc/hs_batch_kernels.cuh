@@ -10,8 +10,8 @@
 // The sums of the FP64 applies (the outer residual ||b - A T||, ||b||, the
 // ABFT checksum sums of the FP64 applies) and the inner solve's starting r.z
 // and r.r are accumulated in FP64 with compensation (hs_csum.h); the inner
-// FP32 iterations' sums are plain FP64 sums of FP32 values.  Every partial is
-// a pair (hi, lo), stored as quantity q and q + NQ, and merged pair-wise.
+// FP32 iterations' sums are plain FP64 sums of FP32 values.  A compensated
+// partial is a pair (hi, lo), stored as quantity q and q + NQ, and merged pair-wise.
 #pragma once
 #include "hs_kernels.cuh"
 #include "hs_csum.h"
