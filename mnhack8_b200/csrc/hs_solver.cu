@@ -382,24 +382,35 @@ const void* pcg_kernel(const hs_solver* h, bool runs) {
         default: return pcg_kernel_form<FORM_FAST>(nk, runs);
     }
 }
+// a run is one flat block up to N = 88; the waits take at most 2 RT tiles
+bool coop_part(const Part& p) { return p.nflat <= UPD_SLOTS && p.nblk <= 2 * RT; }
+// the largest cooperative tile's shared memory
+size_t pcg_smem_most() {
+    size_t most = 0;
+    Part p{};
+    for (int N = 1; (p = make_part(N)).nflat <= UPD_SLOTS; ++N)
+        if (coop_part(p)) most = std::max(most, pcg_smem(p.CX));
+    return most;
+}
 // CTAs of the cooperative solve: one per tile and per run (or per kPcgRuns runs)
 // where they are all resident at once; else 0 (the graph's while loop)
 hs_status set_coop_grid(hs_solver* h, int dev) {
     h->coop_grid = 0;
     if (h->opt.scatter != HS_SCATTER_COLORED || !graphs_enabled() || pdl_enabled()) return HS_OK;
-    // a run is one flat block up to N = 88; the waits take at most 2 RT tiles
-    if (h->part.nflat > UPD_SLOTS || h->part.nblk > 2 * RT) return HS_OK;
+    if (!coop_part(h->part)) return HS_OK;
     const size_t smem = pcg_smem(h->part.CX);
+    static const size_t limit = pcg_smem_most();
     int can = 0, most = 0;
     HS_CUDA(cudaDeviceGetAttribute(&can, cudaDevAttrCooperativeLaunch, dev));
     HS_CUDA(cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-    if (!can || smem + 4096 > (size_t)most) return HS_OK;
+    if (!can || limit + 4096 > (size_t)most) return HS_OK;
     for (const bool runs : {false, true}) {
         const long long nf = h->part.nflat;
         const long long grid = std::max(h->part.ntiles, runs ? (nf + kPcgRuns - 1) / kPcgRuns : nf);
         int per_sm = 0;
         const void* k = pcg_kernel(h, runs);
-        HS_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        // the limit is the kernel's, shared by all handles: always the largest tile's, never this handle's
+        HS_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)limit));
         HS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, ST, smem));
         if ((long long)per_sm * h->n_sm < grid) continue;
         h->coop_grid = (int)grid;
