@@ -869,8 +869,13 @@ hs_status need_T0(hs_solver* h) {
     if (h->T0.p) return HS_OK;
     std::vector<double> v(h->Nn, 0.0);
     if (h->opt.ic_mode == 1) gaussian_ic(h->N, h->opt.ic_sigma, v.data());
-    HS_CUDA(h->T0.alloc(h->Nn));
-    HS_CUDA(cudaMemcpy(h->T0.p, v.data(), h->Nn * 8, cudaMemcpyHostToDevice));
+    DevBuf<double> t;
+    HS_CUDA(t.alloc(h->Nn));
+    // on the handle's own stream: the default stream orders nothing before it
+    // (a copy from pageable memory may still be on its way when it returns)
+    HS_CUDA(cudaMemcpyAsync(t.p, v.data(), h->Nn * 8, cudaMemcpyHostToDevice, h->s));
+    HS_CUDA(cudaStreamSynchronize(h->s));
+    std::swap(h->T0.p, t.p); std::swap(h->T0.n, t.n);       // kept once it is there
     return HS_OK;
 }
 }  // namespace
