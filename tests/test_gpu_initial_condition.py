@@ -1,6 +1,7 @@
 """The initial condition a handle keeps on the device is uploaded on the handle's
 own stream, complete before the first step reads it: a solve neither waits for
-work that the caller has on the default stream nor takes part in its order."""
+work that the caller has on the default stream nor takes part in its order.  A
+trajectory's run keeps it only where that is little memory."""
 import numpy as np
 import pytest
 
@@ -54,3 +55,24 @@ def test_first_run_equals_the_next(N):
     got = h.run_case(2, snap_every=0)["T"]
     assert np.array_equal(bits(first), bits(got))
     h.close()
+
+
+def test_run_case_keeps_no_large_field():
+    """Where device memory is short, a run leaves the handle with what it had
+    (N = 200: 65 MB a field, 3 GB free)."""
+    import torch
+
+    N = 200
+    r = np.ones(N ** 3)
+    g = _lib.Solver(N, 5e-4, r, r, detect=False, no_source=True, ic="gaussian", ic_sigma=0.15)
+    g.advance(1)                                # the graph and its launch are in memory
+    torch.cuda.synchronize()
+    rest = torch.empty(torch.cuda.mem_get_info()[0] - (3 << 30), dtype=torch.uint8, device="cuda")
+    before = torch.cuda.mem_get_info()[0]
+    T = g.run_case(1, snap_every=0)["T"]
+    assert before - torch.cuda.mem_get_info()[0] < 16 << 20
+    del rest
+    torch.cuda.empty_cache()
+    g.advance(1, from_ic=True)                  # this call keeps it, as documented
+    assert np.array_equal(bits(T), bits(g.get_field()))
+    g.close()
