@@ -12,6 +12,7 @@
 #include <vector>
 
 #include "../../include/heat_b200.h"
+#include "hs_grow.h"
 #include "hs_host.h"
 #include "hs_kernels.cuh"
 #include "hs_pcg.cuh"
@@ -49,20 +50,12 @@ struct DevBuf {
 
 // Page-locked host memory that kernels write their results into, so that a call
 // ends with one synchronisation and no copy; kept by the handle and grown on demand
-template <class T>
-struct PinBuf {
-    T* p = nullptr;
-    size_t n = 0;
-    cudaError_t need(size_t count) {
-        if (count <= n) return cudaSuccess;
-        if (p) cudaFreeHost(p);
-        p = nullptr; n = 0;
-        const cudaError_t e = cudaMallocHost(&p, count * sizeof(T));
-        if (e == cudaSuccess) n = count;
-        return e;
-    }
-    ~PinBuf() { if (p) cudaFreeHost(p); }
+struct PinMem {
+    static constexpr cudaError_t ok = cudaSuccess;
+    static cudaError_t get(void** p, size_t bytes) { return cudaMallocHost(p, bytes); }
+    static void put(void* p) { cudaFreeHost(p); }
 };
+template <class T> using PinBuf = GrowBuf<T, PinMem>;
 
 // CUDA events, kept by the handle
 struct Events {
@@ -163,6 +156,8 @@ namespace {
 // room for the results of n steps
 hs_status need_out(hs_solver* h, int n) {
     const size_t m = (size_t)std::max(n, 64);
+    // an earlier call that failed may have left kernels that write there
+    if (m > h->it_out.n || m * 8 > h->rec_out.n) HS_CUDA(cudaStreamSynchronize(h->s));
     HS_CUDA(h->it_out.need(m));
     HS_CUDA(h->rec_out.need(m * 8));
     return HS_OK;
