@@ -28,6 +28,7 @@ void set_error(const std::string& msg) { g_err = msg; }
     do {                                                                                  \
         cudaError_t _e = (call);                                                          \
         if (_e != cudaSuccess) {                                                          \
+            cudaGetLastError();           /* reported here, not by a later call */       \
             hs::set_error(std::string("CUDA error: ") + cudaGetErrorString(_e) + " at " + \
                           __FILE__ + ":" + std::to_string(__LINE__));                    \
             return HS_ERR_CUDA;                                                           \
