@@ -118,6 +118,9 @@ hs_status hs_load_fields(const char* prefix, int N, double* k_out, double* rhoc_
 hs_status hs_create(const hs_options* opt, const double* k_host, const double* rhoc_host, hs_solver** out);
 void      hs_destroy(hs_solver* s);
 long long hs_num_nodes(const hs_solver* s);
+/* CTAs of the one cooperative kernel that a whole PCG solve of this handle is,
+ * or 0 where the solve is a loop of launches (large grids, atomic scatter). */
+int       hs_coop_ctas(const hs_solver* s);
 /* kmin, kmax, rhocmin, rhocmax and the five reference-matrix check errors */
 hs_status hs_field_stats(const hs_solver* s, double out9[9]);
 

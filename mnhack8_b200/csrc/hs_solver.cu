@@ -110,6 +110,7 @@ struct hs_solver {
     int n_sm = 148;
     DevBuf<unsigned> ticket;            // [0] last-CTA tickets; [64], [96] gates of the cooperative solve
     int coop_grid = 0;                  // CTAs of the cooperative solve (k_pcg); 0: the graph's while loop instead
+    const void* coop_kernel = nullptr;  // its instantiation
     XWord* xwords = nullptr;            // its exchange words (in upart)
     unsigned pcg_launches = 0;
     DevBuf<DevState> st;
@@ -402,6 +403,8 @@ hs_status set_coop_grid(hs_solver* h, int dev) {
     if (!can || limit + 4096 > (size_t)most) return HS_OK;
     for (const bool runs : {false, true}) {
         const long long nf = h->part.nflat;
+        // several runs a CTA are for grids of more runs than tiles; else both are the same grid
+        if (runs && nf <= h->part.ntiles) break;
         const long long grid = std::max(h->part.ntiles, runs ? (nf + kPcgRuns - 1) / kPcgRuns : nf);
         int per_sm = 0;
         const void* k = pcg_kernel(h, runs);
@@ -410,6 +413,7 @@ hs_status set_coop_grid(hs_solver* h, int dev) {
         HS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, ST, smem));
         if ((long long)per_sm * h->n_sm < grid) continue;
         h->coop_grid = (int)grid;
+        h->coop_kernel = k;
         break;
     }
     return HS_OK;
@@ -431,7 +435,7 @@ hs_status launch_pcg(hs_solver* h, bool with_rhs) {
     a.d1 = h->opt.detect != 0;
     a.ec = h->ec;
     void* args[] = {&a};
-    HS_CUDA(cudaLaunchCooperativeKernel(pcg_kernel(h, h->coop_grid < a.nruns), dim3(h->coop_grid), dim3(ST), args, pcg_smem(h->part.CX), h->s));
+    HS_CUDA(cudaLaunchCooperativeKernel(h->coop_kernel, dim3(h->coop_grid), dim3(ST), args, pcg_smem(h->part.CX), h->s));
     return HS_OK;
 }
 // a step's iteration count as k_step_end stores it: -1 where a kernel gave up a
@@ -721,6 +725,7 @@ hs_status hs_create(const hs_options* opt, const double* k_host, const double* r
 void hs_destroy(hs_solver* s) { delete s; }
 
 long long hs_num_nodes(const hs_solver* s) { return s ? s->Nn : 0; }
+int hs_coop_ctas(const hs_solver* s) { return s ? s->coop_grid : 0; }
 
 hs_status hs_field_stats(const hs_solver* s, double out9[9]) {
     if (!s || !out9) return HS_ERR_ARG;
