@@ -121,6 +121,10 @@ long long hs_num_nodes(const hs_solver* s);
 /* CTAs of the one cooperative kernel that a whole PCG solve of this handle is,
  * or 0 where the solve is a loop of launches (large grids, atomic scatter). */
 int       hs_coop_ctas(const hs_solver* s);
+/* Kernels wait for their other warps and CTAs for some seconds at most, then
+ * give up, and the call returns HS_ERR_CUDA.  on != 0: every such wait of this
+ * handle counts as given up (for tests of a program's error handling). */
+hs_status hs_fail_waits(hs_solver* s, int on);
 /* kmin, kmax, rhocmin, rhocmax and the five reference-matrix check errors */
 hs_status hs_field_stats(const hs_solver* s, double out9[9]);
 

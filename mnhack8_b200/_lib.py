@@ -22,7 +22,7 @@ STATUS = {0: "HS_OK", 1: "HS_ERR_ARG", 2: "HS_ERR_MATRIX", 3: "HS_ERR_IO", 4: "H
 # every function the header declares (checked by the CPU tests)
 EXPORTS = [
     "hs_default_options", "hs_last_error", "hs_api_version", "hs_get_layout", "hs_load_fields", "hs_create",
-    "hs_destroy", "hs_num_nodes", "hs_coop_ctas", "hs_field_stats", "hs_apply", "hs_precond", "hs_build_rhs", "hs_dot", "hs_pcg",
+    "hs_destroy", "hs_num_nodes", "hs_coop_ctas", "hs_fail_waits", "hs_field_stats", "hs_apply", "hs_precond", "hs_build_rhs", "hs_dot", "hs_pcg",
     "hs_arm_fi", "hs_run_case", "hs_verify", "hs_solve_host", "hs_diag_cg", "hs_set_dump", "hs_set_case_tag",
     "hs_target_on_boundary", "hs_classify", "hs_cli_main", "hs_advance", "hs_set_field", "hs_get_field",
     "hs_time_kernel", "hs_dot_noalloc", "hs_campaign", "hs_batch_default_options", "hs_batch_create",
@@ -118,6 +118,8 @@ def lib():
     L.hs_num_nodes.argtypes = [vp]
     L.hs_coop_ctas.restype = i
     L.hs_coop_ctas.argtypes = [vp]
+    L.hs_fail_waits.restype = i
+    L.hs_fail_waits.argtypes = [vp, i]
     L.hs_field_stats.restype = i
     L.hs_field_stats.argtypes = [vp, vp]
     L.hs_apply.restype = i
@@ -270,6 +272,10 @@ class Solver:
         """CTAs of the one cooperative kernel a whole PCG solve is, or 0 where it
         is a loop of launches."""
         return lib().hs_coop_ctas(self._h)
+
+    def fail_waits(self, on):
+        """Every wait inside a kernel counts as given up (for tests)."""
+        check(lib().hs_fail_waits(self._h, int(on)))
 
     def stats(self):
         out = np.zeros(9)

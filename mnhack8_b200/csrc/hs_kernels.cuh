@@ -310,9 +310,10 @@ struct ApplyArgs {
     const double* F;        // ROLE_RHS source (null: none)
     double dtF;
     int d1;                 // evaluate the D1 checksum
-    int pad1;
+    int fail_waits;         // every wait counts as given up (tests)
     double* partials;
     DevState* st;
+    unsigned* gave_up;      // page-locked host word: a wait gave up
     ElemConsts ec;
 };
 
@@ -356,6 +357,7 @@ struct __align__(16) SlabSmem {
     double2 Y3[SPOS];       // from the element at position j-Cw-1:   (q3, q7)
     double sh[MAXQ][8];
     unsigned long long free_bar;
+    unsigned bad;           // a wait gave up
 };
 __device__ __forceinline__ void mbar_init(unsigned b, unsigned n) {
     asm volatile("mbarrier.init.shared.b64 [%0], %1;" ::"r"(b), "r"(n) : "memory");
@@ -364,10 +366,14 @@ __device__ __forceinline__ void mbar_inval(unsigned b) { asm volatile("mbarrier.
 __device__ __forceinline__ void mbar_arrive(unsigned b) {
     asm volatile("{\n\t.reg .b64 t;\n\tmbarrier.arrive.shared.b64 t, [%0];\n\t}" ::"r"(b) : "memory");
 }
+// Polls of a wait before it gives up: seconds, where a legitimate wait lasts as
+// long as one phase of the slowest warp or CTA.  A kernel that gives up says so
+// in a word of the host's, which every call looks at after its synchronisation.
+constexpr unsigned kPolls = 1u << 22;
 // Waits for the phase of parity `phase`, in which every warp of the CTA arrives;
-// false after about a second
+// false: gave up
 __device__ __forceinline__ bool mbar_wait(unsigned b, unsigned phase) {
-    unsigned ok = 0, left = 1u << 22;
+    unsigned ok = 0, left = kPolls;
     do {
         asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
                      : "=r"(ok) : "r"(b), "r"(phase) : "memory");
@@ -454,6 +460,11 @@ __device__ __forceinline__ void slab_march(const ApplyArgs& a, SlabSmem& S, cons
     const int lane = tid & 31;
     const unsigned free_bar = (unsigned)__cvta_generic_to_shared(&S.free_bar);
     unsigned phase = 0;
+    // the hand-over buffers are free again; a CTA that gives up the wait runs on
+    // (its accesses do not depend on what it read), says so at the end, and the call fails
+    auto wait_free = [&]() {
+        if (!mbar_wait(free_bar, phase)) S.bad = 1u;
+    };
     // ac: node sums of plane ix from layer ix-1.  P0, P1, P2: shared planes ix, ix+1, ix+2.
     double ac[SK], an[SK];
     auto layer = [&](int ix, double* P0, double* P1, double* P2) {
@@ -479,7 +490,7 @@ __device__ __forceinline__ void slab_march(const ApplyArgs& a, SlabSmem& S, cons
                 if (fi_r && (long long)ix * eplane + G.eoff[k] == fi_elem) v[0] = flipbit(v[0], fi_bit);
                 ac[k] = dadd(ac[k], v[0]);
                 an[k] = dadd(0.0, v[4]);
-                if (k == 0 && ix >= xa && !mbar_wait(free_bar, phase)) a.st->stuck = 1;   // the hand-over buffers are free again
+                if (k == 0 && ix >= xa) wait_free();
                 if (ev) {
                     S.Y1[j + 1] = make_double2(v[1], v[5]);
                     S.Y2[j + Cw] = make_double2(v[2], v[6]);
@@ -489,7 +500,7 @@ __device__ __forceinline__ void slab_march(const ApplyArgs& a, SlabSmem& S, cons
         } else {
 #pragma unroll
             for (int k = 0; k < SK; ++k) an[k] = 0.0;
-            if (ix >= xa && !mbar_wait(free_bar, phase)) a.st->stuck = 1;
+            if (ix >= xa) wait_free();
         }
         if (ix >= xa) phase ^= 1u;
         ld_coef(ix + 1 <= xb ? ix + 1 : -1);
@@ -523,7 +534,7 @@ __device__ __forceinline__ void slab_march(const ApplyArgs& a, SlabSmem& S, cons
         if (MODE == 0) ld_f(ix + 1);
     };
 
-    if (tid == 0) mbar_init(free_bar, ST / 32);
+    if (tid == 0) { mbar_init(free_bar, ST / 32); S.bad = 0u; }
     double *P0 = S.P[0], *P1 = S.P[1], *P2 = S.P[2];
 #pragma unroll
     for (int k = 0; k < SK; ++k) ac[k] = 0.0;
@@ -543,7 +554,10 @@ __device__ __forceinline__ void slab_march(const ApplyArgs& a, SlabSmem& S, cons
         double* t = P0; P0 = P1; P1 = P2; P2 = t;
     }
     __syncthreads();
-    if (tid == 0) mbar_inval(free_bar);
+    if (tid == 0) {
+        mbar_inval(free_bar);
+        if (S.bad || a.fail_waits) { a.st->stuck = 1; *a.gave_up = 1u; }
+    }
 }
 
 // Colored operator: tile blockIdx.x of the slab partition (every node of the
@@ -647,7 +661,7 @@ __device__ __forceinline__ void update_scalars(const UpdateArgs& a, const double
         st->rho = part[1];
         st->rel0 = __ddiv_rn(__dsqrt_rn(part[2]), bnorm);
         st->iter = 0; st->broken = 0; st->result = 0; st->beta = 0.0;
-        st->done = (st->max_iter <= 0) ? 1 : 0;
+        st->done = (st->max_iter <= 0 || st->stuck) ? 1 : 0;
         st->x_pend = 0;
     } else {
         const int iter = st->iter;
@@ -667,6 +681,7 @@ __device__ __forceinline__ void update_scalars(const UpdateArgs& a, const double
             st->iter = iter + 1;
             if (iter + 1 >= st->max_iter) { st->done = 1; st->result = st->max_iter; }
         }
+        if (st->stuck) st->done = 1;            // an operator gave up a wait: the call fails
         if (a.use_cond) cudaGraphSetConditional(a.cond, st->done ? 0u : 1u);
     }
 }
@@ -1213,7 +1228,7 @@ __global__ void k_step_begin(DevState* st, StepCtl c, double* T, unsigned* count
 __global__ void k_disarm_R(DevState* st) { st->fi_armR = 0; }
 __global__ void k_step_end(DevState* st, int* iters_out, double* d1_out, double* d1_last_out) {
     st->fi_armR = 0; st->fi_vec = 0;
-    *iters_out = st->stuck ? -1 : st->result;
+    *iters_out = st->result;
     *d1_out = st->d1_step;
     if (d1_last_out) *d1_last_out = st->d1_last;
 }

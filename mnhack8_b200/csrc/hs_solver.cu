@@ -123,8 +123,10 @@ struct hs_solver {
     double tol = 0;
 
     // results written by kernels (k_step_end and the detectors), and timing events
-    PinBuf<int> it_out;                 // per step: CG iterations (-1: a wait gave up)
+    PinBuf<int> it_out;                 // per step: CG iterations
     PinBuf<double> rec_out;             // per step: d1, d2, tmin, tmax, E, spread, d1 of the last apply
+    PinBuf<unsigned> gave_up;           // a kernel gave up a wait (check_waits)
+    bool fail_waits = false;            // every wait counts as given up (hs_fail_waits)
     Events ev;
 
     // PCG graphs built on first use: [0] step (RHS + PCG), [1] PCG only
@@ -158,6 +160,10 @@ namespace {
 // room for the results of n steps
 hs_status need_out(hs_solver* h, int n) {
     const size_t m = (size_t)std::max(n, 64);
+    if (!h->gave_up.p) {
+        HS_CUDA(h->gave_up.need(1));
+        *h->gave_up.p = 0u;
+    }
     // an earlier call that failed may have left kernels that write there
     if (m > h->it_out.n || m * 8 > h->rec_out.n) HS_CUDA(cudaStreamSynchronize(h->s));
     HS_CUDA(h->it_out.need(m));
@@ -259,6 +265,7 @@ ApplyArgs colored_args(hs_solver* h, int role, const double* x, double* y, doubl
     a.y = y; a.coef = h->coef.p; a.kc = h->kc.p; a.rc = h->rhocmin; a.w = w; a.F = F; a.dtF = dtF;
     a.d1 = d1 ? 1 : 0;
     a.partials = h->partials.p; a.st = h->st.p; a.ec = h->ec;
+    a.fail_waits = h->fail_waits; a.gave_up = h->gave_up.p;
     return a;
 }
 
@@ -433,17 +440,18 @@ hs_status launch_pcg(hs_solver* h, bool with_rhs) {
     a.with_rhs = with_rhs ? 1 : 0;
     a.nruns = update_runs(h);
     a.d1 = h->opt.detect != 0;
+    a.fail_waits = h->fail_waits; a.gave_up = h->gave_up.p;
     a.ec = h->ec;
     void* args[] = {&a};
     HS_CUDA(cudaLaunchCooperativeKernel(h->coop_kernel, dim3(h->coop_grid), dim3(ST), args, pcg_smem(h->part.CX), h->s));
     return HS_OK;
 }
-// a step's iteration count as k_step_end stores it: -1 where a kernel gave up a
-// wait (DevState::stuck)
-hs_status check_iters(const int* it, int n) {
-    for (int i = 0; i < n; ++i)
-        if (it[i] < 0) { set_error("a kernel gave up waiting for its other warps or blocks"); return HS_ERR_CUDA; }
-    return HS_OK;
+// after a call's synchronisation: did a kernel give up a wait?
+hs_status check_waits(hs_solver* h) {
+    if (!*h->gave_up.p) return HS_OK;
+    *h->gave_up.p = 0u;
+    set_error("a kernel gave up waiting for its other warps or blocks");
+    return HS_ERR_CUDA;
 }
 
 // build a graph: [rhs] + x0 matvec + prologue, then while(!done){ (K1; K2) x kLoopUnroll }.
@@ -727,6 +735,17 @@ void hs_destroy(hs_solver* s) { delete s; }
 long long hs_num_nodes(const hs_solver* s) { return s ? s->Nn : 0; }
 int hs_coop_ctas(const hs_solver* s) { return s ? s->coop_grid : 0; }
 
+hs_status hs_fail_waits(hs_solver* s, int on) {
+    if (!s) return HS_ERR_ARG;
+    s->fail_waits = on != 0;
+    for (int i = 0; i < 2; ++i) {               // the graphs hold what they were built with
+        if (s->gexec[i]) cudaGraphExecDestroy(s->gexec[i]);
+        if (s->graph[i]) cudaGraphDestroy(s->graph[i]);
+        s->gexec[i] = nullptr; s->graph[i] = nullptr;
+    }
+    return HS_OK;
+}
+
 hs_status hs_field_stats(const hs_solver* s, double out9[9]) {
     if (!s || !out9) return HS_ERR_ARG;
     out9[0] = s->kmin; out9[1] = s->kmax; out9[2] = s->rhocmin; out9[3] = s->rhocmax;
@@ -775,7 +794,7 @@ hs_status hs_apply(hs_solver* s, const double* x, double* y, double dt_eff, int 
     k_step_end<<<1, 1, 0, s->s>>>(s->st.p, s->it_out.p, s->rec_out.p, s->rec_out.p + 6);
     HS_CUDA(cudaGetLastError());
     HS_CUDA(cudaStreamSynchronize(s->s));
-    const hs_status st = check_iters(s->it_out.p, 1);
+    const hs_status st = check_waits(s);
     if (st != HS_OK) return st;
     if (d1 && abft_rel) *abft_rel = s->rec_out.p[6];
     return HS_OK;
@@ -797,7 +816,7 @@ hs_status hs_build_rhs(hs_solver* s, const double* T, double* b) {
     apply_projected(s, ROLE_RHS, T, b, 0.0, d1, s->wM.p, src ? s->F.p : nullptr, s->opt.dt);
     HS_CUDA(cudaGetLastError());
     HS_CUDA(cudaStreamSynchronize(s->s));
-    return HS_OK;
+    return check_waits(s);
 }
 
 hs_status hs_dot(hs_solver* s, const double* x, const double* y, double* out) {
@@ -928,7 +947,7 @@ hs_status hs_pcg(hs_solver* s, const double* b, double* x, int max_iter, double 
     HS_CUDA(cudaGetLastError());
     HS_CUDA(cudaMemcpyAsync(x, s->T.p, s->Nn * 8, cudaMemcpyDeviceToDevice, s->s));
     HS_CUDA(cudaStreamSynchronize(s->s));
-    st = check_iters(s->it_out.p, 1);
+    st = check_waits(s);
     if (st != HS_OK) return st;
     if (iters) *iters = s->it_out.p[0];
     return HS_OK;
@@ -1044,7 +1063,7 @@ hs_status run_case_impl(hs_solver* h, int n_steps, int snap_every, const hs_fi_s
     HS_CUDA(cudaStreamSynchronize(h->s));
     const int* it = h->it_out.p;
     const double* rec = h->rec_out.p;
-    st = check_iters(it + s0, n_steps - s0);
+    st = check_waits(h);
     if (st != HS_OK) return st;
     int nf = 0;
     si = 0;
@@ -1104,7 +1123,7 @@ hs_status hs_verify(hs_solver* h, int n_steps, double* rel_err, long long* total
     float fms = 0.f;
     HS_CUDA(cudaEventElapsedTime(&fms, e0, e1));
     const int* it = h->it_out.p;
-    st = check_iters(it, n_steps);
+    st = check_waits(h);
     if (st != HS_OK) return st;
     long long tot = 0;
     for (int i = 0; i < n_steps; ++i) tot += it[i];
@@ -1146,7 +1165,7 @@ hs_status hs_solve_host(hs_solver* h, const double* T0_host, double* T_host, int
     float fms = 0.f;
     HS_CUDA(cudaEventElapsedTime(&fms, e0, e1));
     const int* it = h->it_out.p;
-    st = check_iters(it, n_steps);
+    st = check_waits(h);
     if (st != HS_OK) return st;
     long long tot = 0;
     for (int i = 0; i < n_steps; ++i) tot += it[i];
@@ -1206,7 +1225,7 @@ hs_status hs_diag_cg(hs_solver* h, int max_iter, double tol, double* rel0, doubl
     if (st != HS_OK) return st;
     HS_CUDA(cudaStreamSynchronize(h->s));
     const int it = h->it_out.p[0];
-    st = check_iters(&it, 1);
+    st = check_waits(h);
     if (st != HS_OK) return st;
     HS_CUDA(cudaMemcpy(&hsx, h->st.p, sizeof(hsx), cudaMemcpyDeviceToHost));
     const int n = std::min(it, cap);
@@ -1262,7 +1281,7 @@ hs_status hs_advance(hs_solver* h, int n_steps, int from_ic, long long* total_it
     float fms = 0.f;
     HS_CUDA(cudaEventElapsedTime(&fms, e0, e1));
     const int* it = h->it_out.p;
-    st = check_iters(it, n_steps);
+    st = check_waits(h);
     if (st != HS_OK) return st;
     long long tot = 0;
     for (int i = 0; i < n_steps; ++i) tot += it[i];
@@ -1321,6 +1340,8 @@ hs_status hs_time_kernel(hs_solver* h, int which, int reps, double* ms_per_launc
     }
     saved.done = 1;
     HS_CUDA(cudaMemcpy(h->st.p, &saved, sizeof(saved), cudaMemcpyHostToDevice));
+    const hs_status st = check_waits(h);
+    if (st != HS_OK) return st;
     if (ms_per_launch) *ms_per_launch = tot / reps;
     return HS_OK;
 }

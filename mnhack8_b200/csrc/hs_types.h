@@ -123,7 +123,7 @@ struct DevState {
     // last update (at x_pend_iter) still owed when the loop ends
     double alpha_hist[2];
     int x_pend, x_pend_iter;
-    int stuck, pad2;        // a kernel gave up a bounded wait
+    int stuck, pad2;        // a kernel of this step gave up a bounded wait: the solve ends
     // scratch outputs of standalone reductions
     double red_out[MAXQ];
     double mm_out[2];       // min, max
