@@ -1213,6 +1213,15 @@ hs_status hs_diag_cg(hs_solver* h, int max_iter, double tol, double* rel0, doubl
     HS_CUDA(lg.alloc((size_t)3 * std::max(cap, 1)));
     DevState hsx{};
     HS_CUDA(cudaMemcpy(&hsx, h->st.p, sizeof(hsx), cudaMemcpyDeviceToHost));
+    // whichever way this call ends, no later solve logs into the buffer it frees
+    struct Unlog {
+        hs_solver* h;
+        ~Unlog() {
+            static_assert(offsetof(DevState, log_cap) == offsetof(DevState, log_rel) + 3 * sizeof(double*), "one range");
+            cudaMemsetAsync(&h->st.p->log_rel, 0, 3 * sizeof(double*) + sizeof(int), h->s);
+            cudaStreamSynchronize(h->s);
+        }
+    } unlog{h};
     hsx.log_rel = lg.p; hsx.log_alpha = lg.p + cap; hsx.log_beta = lg.p + 2 * cap; hsx.log_cap = cap;
     HS_CUDA(cudaMemcpy(h->st.p, &hsx, sizeof(hsx), cudaMemcpyHostToDevice));
     // one solve from the initial condition, no fault, no detector bookkeeping
@@ -1234,8 +1243,6 @@ hs_status hs_diag_cg(hs_solver* h, int max_iter, double tol, double* rel0, doubl
     if (beta && n) HS_CUDA(cudaMemcpy(beta, lg.p + 2 * cap, n * 8, cudaMemcpyDeviceToHost));
     if (rel0) *rel0 = hsx.rel0;
     if (iters) *iters = it;
-    hsx.log_rel = hsx.log_alpha = hsx.log_beta = nullptr; hsx.log_cap = 0;
-    HS_CUDA(cudaMemcpy(h->st.p, &hsx, sizeof(hsx), cudaMemcpyHostToDevice));
     return HS_OK;
 }
 

@@ -60,3 +60,20 @@ def test_atomic_scatter_has_no_waits():
     g.fail_waits(True)
     g.run_case(1, snap_every=0)
     g.close()
+
+
+@pytest.mark.parametrize("N", [12, 80])
+def test_failed_log_leaves_nothing_behind(N):
+    """A diag_cg that fails frees the buffer its solve logged into; later solves
+    of the handle give what they gave, and a later log is whole."""
+    g = solver(N, "wht")
+    n, log = g.diag_cg()
+    want = g.run_case(2, snap_every=0)["T"]
+    g.fail_waits(True)
+    with pytest.raises(_lib.HeatError, match="gave up"):
+        g.diag_cg()
+    g.fail_waits(False)
+    assert np.array_equal(bits(g.run_case(2, snap_every=0)["T"]), bits(want))
+    m, again = g.diag_cg()
+    assert m == n and all(np.array_equal(bits(again[k]), bits(log[k])) for k in ("rel", "alpha", "beta"))
+    g.close()
