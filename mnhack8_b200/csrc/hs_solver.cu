@@ -157,6 +157,12 @@ struct hs_solver {
 
 namespace {
 
+// the handle's state from the host, in place when this returns (on the handle's
+// stream: the default stream orders nothing before it)
+cudaError_t put_state(hs_solver* h, const DevState& v) {
+    const cudaError_t e = cudaMemcpyAsync(h->st.p, &v, sizeof(v), cudaMemcpyHostToDevice, h->s);
+    return e == cudaSuccess ? cudaStreamSynchronize(h->s) : e;
+}
 // room for the results of n steps
 hs_status need_out(hs_solver* h, int n) {
     const size_t m = (size_t)std::max(n, 64);
@@ -718,7 +724,7 @@ hs_status hs_create(const hs_options* opt, const double* k_host, const double* r
         HS_CUDA(cudaMemcpy(&hs, h->st.p, sizeof(hs), cudaMemcpyDeviceToHost));
         hs.norm_wM = std::sqrt(nr[0]);
         hs.norm_wA = std::sqrt(nr[2]);
-        HS_CUDA(cudaMemcpy(h->st.p, &hs, sizeof(hs), cudaMemcpyHostToDevice));
+        HS_CUDA(put_state(h.get(), hs));
         HS_CUDA(cudaMemsetAsync(h->r.p, 0, Nn * 8, h->s));
     }
     HS_CUDA(cudaStreamSynchronize(h->s));
@@ -1223,7 +1229,7 @@ hs_status hs_diag_cg(hs_solver* h, int max_iter, double tol, double* rel0, doubl
         }
     } unlog{h};
     hsx.log_rel = lg.p; hsx.log_alpha = lg.p + cap; hsx.log_beta = lg.p + 2 * cap; hsx.log_cap = cap;
-    HS_CUDA(cudaMemcpy(h->st.p, &hsx, sizeof(hsx), cudaMemcpyHostToDevice));
+    HS_CUDA(put_state(h, hsx));
     // one solve from the initial condition, no fault, no detector bookkeeping
     std::vector<double> T0(h->Nn, 0.0);
     if (h->opt.ic_mode == 1) gaussian_ic(h->N, h->opt.ic_sigma, T0.data());
@@ -1306,7 +1312,7 @@ hs_status hs_time_kernel(hs_solver* h, int which, int reps, double* ms_per_launc
     hsx.done = 0; hsx.broken = 0; hsx.iter = 1; hsx.beta = 0.5; hsx.rho = 1.0; hsx.alpha = 1e-3;
     hsx.bnorm = 1.0; hsx.tol = 0.0; hsx.max_iter = 1 << 30; hsx.fi_armR = 0; hsx.fi_vec = 0;
     hsx.log_rel = hsx.log_alpha = hsx.log_beta = nullptr; hsx.log_cap = 0;
-    HS_CUDA(cudaMemcpy(h->st.p, &hsx, sizeof(hsx), cudaMemcpyHostToDevice));
+    HS_CUDA(put_state(h, hsx));
     // nonzero, SPD-consistent inputs (p.Ap > 0): the positive diagonal
     for (double* v : {h->z.p, h->p0.p, h->p1.p, h->T.p, h->r.p})
         k_copy<<<grid_for(h->Nn, RT), RT, 0, h->s>>>(h->Nn, h->diag.p, v);
@@ -1346,7 +1352,7 @@ hs_status hs_time_kernel(hs_solver* h, int which, int reps, double* ms_per_launc
         tot += ms;
     }
     saved.done = 1;
-    HS_CUDA(cudaMemcpy(h->st.p, &saved, sizeof(saved), cudaMemcpyHostToDevice));
+    HS_CUDA(put_state(h, saved));
     const hs_status st = check_waits(h);
     if (st != HS_OK) return st;
     if (ms_per_launch) *ms_per_launch = tot / reps;
