@@ -354,11 +354,18 @@ hs_status batch_add_impl(hs_batch* b, int N, double dt, const double* k, const d
     HS_CUDA(cudaSetDevice(b->opt.device));
     const long long NN = N + 1, Nn = NN * NN * NN, Ne = (long long)N * N * N;
     bool uniform = true;            // rho*c is one value
-    if (!gen)
-        for (long long e = 0; e < Ne; ++e) {
+    if (!gen) {
+        // as long as rho*c is its first value, comparing with that is its check:
+        // two comparisons an element either way (an admission at N=96 takes 2.0 ms
+        // with two, 2.5 with three)
+        long long e = 0;
+        if (rhoc[0] > 0)
+            for (; e < Ne; ++e)
+                if (!(k[e] > 0) || rhoc[e] != rhoc[0]) break;
+        uniform = e == Ne;
+        for (; e < Ne; ++e)
             if (!(k[e] > 0) || !(rhoc[e] > 0)) { set_error("hs_batch_add: non-positive coefficient"); return HS_ERR_ARG; }
-            uniform = uniform && rhoc[e] == rhoc[0];
-        }
+    }
     const RefMatrices mats = build_reference_matrices(N);
     if (!mats.ok) { set_error("reference-matrix self-check failed"); return HS_ERR_MATRIX; }
     // slot
