@@ -27,9 +27,13 @@ void gaussian_ic(int N, double sigma, double* T);
 void exact_mode(int N, double t, double alpha, double* v);
 
 // Make the pages of a host buffer that a field is about to be copied into
-// resident (values unchanged), on several threads where that is worth it.  A
-// copy into fresh pages takes its page faults one by one inside the driver: a
-// 136 MB field 66 ms, 7 ms once the pages are there.
+// resident (values unchanged).  A copy into fresh pages takes its page faults one
+// by one inside the driver: a 136 MB field 29 ms, 12 with this (7 where the pages
+// are there).  parallel: the caller waits meanwhile, so several threads share the
+// work, from 32 MB on: smaller buffers mostly have their pages (malloc hands them
+// out again from its heap), and the threads then only cost time (read-back at
+// N = 64, 2.2 MB: 157 us, 208 with threads).  Else one thread, from 1 MB on,
+// behind work that the device is doing.
 void touch_pages(void* p, size_t bytes, bool parallel);
 
 void set_error(const std::string& msg);

@@ -209,15 +209,15 @@ void exact_mode(int N, double t, double alpha, double* v) {
 }
 
 void touch_pages(void* p, size_t bytes, bool parallel) {
-    constexpr size_t kPage = 4096, kLeast = (size_t)1 << 20;
-    if (bytes < kLeast) return;
+    constexpr size_t kPage = 4096, kMiB = (size_t)1 << 20;
+    if (bytes < (parallel ? 32 * kMiB : kMiB)) return;
     unsigned char* const c = static_cast<unsigned char*>(p);
     // one store per page that leaves the byte as it is, whoever else reads it meanwhile
     auto touch = [=](size_t a, size_t b) {
         for (size_t i = a; i < b; ++i) __atomic_fetch_or(c + i * kPage, (unsigned char)0, __ATOMIC_RELAXED);
     };
     const size_t n = (bytes + kPage - 1) / kPage;       // the last page through its part of the buffer
-    const size_t nt = parallel ? std::min<size_t>(bytes < 4 * kLeast ? 4 : 8, (size_t)hw_threads()) : 1;
+    const size_t nt = parallel ? std::min<size_t>(8, (size_t)hw_threads()) : 1;
     std::vector<std::thread> th;
     size_t next = 0;
     try {

@@ -74,12 +74,12 @@ struct Events {
     ~Events() { for (auto v : e) cudaEventDestroy(v); }
 };
 
-// touch_pages for a caller's output buffer; a device address is left to the
-// copy, which refuses it
+// touch_pages for a caller's output buffer in ordinary memory: page-locked pages
+// are resident, managed ones may be the device's, and device memory is the copy's
 void touch_output(void* p, size_t bytes, bool parallel) {
     cudaPointerAttributes at{};
     if (cudaPointerGetAttributes(&at, p) != cudaSuccess) { cudaGetLastError(); return; }
-    if (at.type != cudaMemoryTypeDevice) touch_pages(p, bytes, parallel);
+    if (at.type == cudaMemoryTypeUnregistered) touch_pages(p, bytes, parallel);
 }
 
 inline int grid_for(long long n, int threads, int cap = 148 * 16) {
