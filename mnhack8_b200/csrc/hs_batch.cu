@@ -467,7 +467,8 @@ hs_status batch_add_impl(hs_batch* b, int N, double dt, const double* k, const d
     sl.used = true; sl.N = N; sl.dt = dt; sl.steps_left = n_steps; sl.steps_done = 0;
     sl.part = batch_part(N, b->opt.tile_planes);
     d.part = sl.part;
-    d.nchunk = (Nn + UC - 1) / UC;
+    d.rounds = upd_rounds(Nn);
+    d.nchunk = (Nn + (long long)d.rounds * UR - 1) / ((long long)d.rounds * UR);
     sl.mem = mem;
     sl.desc = d;
     b->dirty = true;

@@ -107,7 +107,7 @@ struct BInst {
     int active;
     int uniform;               // rho*c is one value: k32 holds k alone
     float rc32;                // and its value
-    int pad;
+    int rounds;                // of the inner update's chunks (upd_rounds)
     double* T;                 // solution (updated in place)
     double* b;                 // right-hand side M T_old
     double* y64;               // FP64 operator output
@@ -374,10 +374,12 @@ __device__ __forceinline__ void cta_tree_w(double (&v)[NQ], double (*sh)[16]) {
     }
 }
 // The CTA's sums become partial idx of an instance's count partials (quantity q
-// at base + q * stride); in the last CTA to get here they are added up (strided
-// sums, then the tree) and true is returned, with the totals in thread 0.
-template <int NQ, int NT, int FB>
-__device__ __forceinline__ bool inst_finish(double (&v)[NQ], double* base, long long stride, long long idx,
+// at base + q * stride); true in the last CTA to get here, which adds them up
+// (inst_total).  The state it needs for its scalar step is read in between: after
+// the totals those loads came one after the other (2 instances at N=16 2.71 -> 2.58
+// ms of 4 steps, one at N=160 28.2 -> 27.3).
+template <int NQ, int NT>
+__device__ __forceinline__ bool inst_arrive(double (&v)[NQ], double* base, long long stride, long long idx,
                                             long long count, unsigned* ticket, double (*sh)[16], unsigned* s_last) {
     cta_tree_w<NQ, NT / 32>(v, sh);
     if (threadIdx.x == 0) {
@@ -389,6 +391,12 @@ __device__ __forceinline__ bool inst_finish(double (&v)[NQ], double* base, long 
     __syncthreads();
     if (!*s_last) return false;
     __threadfence();
+    return true;
+}
+// strided sums of the instance's partials, then the tree: the totals in thread 0
+template <int NQ, int NT, int FB>
+__device__ __forceinline__ void inst_total(double (&v)[NQ], const double* base, long long stride, long long count,
+                                           unsigned* ticket, double (*sh)[16]) {
 #pragma unroll
     for (int q = 0; q < NQ; ++q) v[q] = 0.0;
     for (long long k0 = threadIdx.x; k0 < count; k0 += (long long)NT * FB) {
@@ -407,7 +415,6 @@ __device__ __forceinline__ bool inst_finish(double (&v)[NQ], double* base, long 
     }
     cta_tree_w<NQ, NT / 32>(v, sh);
     if (threadIdx.x == 0) *ticket = 0u;
-    return true;
 }
 
 // Two FP32 lanes in one 64-bit register, each rounded like the scalar operation.
@@ -663,17 +670,22 @@ __global__ void __launch_bounds__(FT, 2) kb_apply32(BatchArgs B) {
         else kb_march32<false, false>(B, S, I, T, part);
     }
     const long long nt = I.part.ntiles;
-    if (!inst_finish<MAXQ, FT, 2>(part, B.pa + I.tile0, B.ntiles, t - I.tile0, nt, &st->tick_a, S.sh, &S.last)) return;
+    double* const base = B.pa + I.tile0;
+    if (!inst_arrive<MAXQ, FT>(part, base, B.ntiles, t - I.tile0, nt, &st->tick_a, S.sh, &S.last)) return;
+    const double nw = __ldcg(&st->norm_wA), d1_max = __ldcg(&st->d1_max32), rho = __ldcg(&st->rho), alpha = __ldcg(&st->alpha);
+    const long long applies = __ldcg(&st->applies32);
+    const int stuck = __ldcg(&st->stuck);
+    inst_total<MAXQ, FT, 2>(part, base, B.ntiles, nt, &st->tick_a, S.sh);
     if (threadIdx.x != 0) return;
     if (B.detect) {
-        const double rel = d1_rel(part, st->norm_wA);
+        const double rel = d1_rel(part, nw);
         st->d1_last = rel;
-        st->d1_max32 = fmax(st->d1_max32, rel);
+        st->d1_max32 = fmax(d1_max, rel);
     }
-    st->applies32 += 1;
-    if (!isfinite(part[0]) || st->stuck) { st->inner_bad = 1; st->done = 1; st->stuck = 0; }
+    st->applies32 = applies + 1;
+    if (!isfinite(part[0]) || stuck) { st->inner_bad = 1; st->done = 1; st->stuck = 0; }
     else if (fabs(part[0]) < 1e-30) { st->broken = 1; st->done = 1; }
-    else { st->alpha_prev = st->alpha; st->alpha = __ddiv_rn(st->rho, part[0]); }
+    else { st->alpha_prev = alpha; st->alpha = __ddiv_rn(rho, part[0]); }
 }
 
 // compensated sums of one instance's partials: count (hi, lo) pairs per
@@ -812,30 +824,32 @@ __global__ void __launch_bounds__(RT) kb_outer_final(BatchArgs B) {
 // r -= alpha Ap, z = r / diag; r.r and r.z; and at odd iterations d += alpha p
 // for the previous iteration and this one (the same two multiply-adds in the
 // same order; the previous p is still in the other buffer), which saves 4 of 32
-// bytes per node on average.  A block takes a chunk of UC consecutive nodes in
-// UL rounds of UV groups of four per thread, a round's loads in flight together;
-// the last block of an instance to finish adds up its chunks' sums and does the
-// inner solve's scalar step (beta, convergence).  The block's tree, fence and
-// ticket are what a chunk must outweigh (24 instances of N 16..96 / N=160, device
-// ms: 1024 nodes 170 / 175, 2048 148 / 148; with d every second iteration at 64
-// registers 2048 150 / 150, 4096 147 / 148, 8192 145 / 145).
-constexpr int UV = 2, UL = 4, UC = RT * 4 * UV * UL;
-__global__ void __launch_bounds__(RT, 4) kb_update32(BatchArgs B) {
-    __shared__ double sh[2][16];
-    __shared__ unsigned s_last;
-    const int slot = B.chunk2inst[blockIdx.x];
-    if (slot < 0) return;
-    const BInst& I = B.inst[slot];
-    BState* st = I.st;
-    if (!I.active || st->odone || st->done) return;
-    const long long chunk = blockIdx.x - I.chunk0, Nn = I.part.Nn;
-    const int iter = st->iter;
+// bytes per node on average.  A block takes a chunk of consecutive nodes in rounds
+// of UR (UV groups of four per thread, a round's loads in flight together); the
+// last block of an instance to finish adds up its chunks' sums and does the inner
+// solve's scalar step (beta, convergence).
+//
+// Rounds per chunk, by the grid alone (so that an instance has the same bits alone
+// and among others): one while that makes at most two blocks per SM (N <= 83), two
+// while all its blocks are resident at once (148 SMs of 4 blocks: N <= 133), else
+// four.  A small instance is bound by latency, and each further round is one more
+// chain of loads on a mostly idle GPU; a large one by the memory, and then by the
+// tree, fence and ticket that each block costs.  Device ms of 4 steps (B200) with
+// one | two | four rounds: 2 instances at N=48 5.20 | 5.40 | 5.83, 16 at N=64 23.9 |
+// 22.8 | 22.3, one at N=96 10.5 | 10.6 | 11.0, 16 at N=96 79.8 | 75.7 | 75.3, one at
+// N=128 15.5 | 14.7 | 15.1, 4 at N=128 56.4 | 54.0 | 52.7.
+constexpr int UV = 2, UR = RT * 4 * UV;
+inline int upd_rounds(long long Nn) {
+    return Nn <= 148ll * 2 * UR ? 1 : Nn <= 148ll * 4 * 2 * UR ? 2 : 4;
+}
+// the chunk's nodes; the thread's r.r and r.z into part
+__device__ __forceinline__ void upd32_chunk(const BInst& I, BState* st, int rounds, long long chunk, double (&part)[2]) {
+    const long long Nn = I.part.Nn;
     const float alpha = (float)st->alpha;
-    const bool odd = iter & 1;
+    const bool odd = st->iter & 1;
     const float alpha_prev = odd ? (float)st->alpha_prev : 0.f;
     const bool fr = fi_now(st, FI_RV);
     const long long fi_idx = fr ? st->fi_idx : -1;
-    double part[2] = {0.0, 0.0};
     // four nodes from m on (the buffers are 256-byte aligned, m a multiple of 4); the end of the grid one by one
     auto ld4 = [&](const float* v, long long m) {
         if (m + 3 < Nn) return *reinterpret_cast<const float4*>(v + m);
@@ -848,8 +862,8 @@ __global__ void __launch_bounds__(RT, 4) kb_update32(BatchArgs B) {
         if (m + 2 < Nn) v[m + 2] = x.z;
     };
     float4 dv[UV], pv[UV], ov[UV], qv[UV], rv[UV], iv[UV];
-    for (int ul = 0; ul < UL; ++ul) {
-        const long long m0 = chunk * UC + ul * (RT * 4 * UV) + threadIdx.x * 4;
+    for (int ul = 0; ul < rounds; ++ul) {
+        const long long m0 = (chunk * rounds + ul) * UR + threadIdx.x * 4;
 #pragma unroll
         for (int u = 0; u < UV; ++u) {
             const long long m = m0 + u * (RT * 4);
@@ -882,16 +896,33 @@ __global__ void __launch_bounds__(RT, 4) kb_update32(BatchArgs B) {
             st4(I.r32, m, rv[u]); st4(I.z32, m, zv);
         }
     }
-    if (!inst_finish<2, RT, 8>(part, B.pf + I.chunk0, B.nflat, chunk, I.nchunk, &st->tick_u, sh, &s_last)) return;
+}
+__global__ void __launch_bounds__(RT, 4) kb_update32(BatchArgs B) {
+    __shared__ double sh[2][16];
+    __shared__ unsigned s_last;
+    const int slot = B.chunk2inst[blockIdx.x];
+    if (slot < 0) return;
+    const BInst& I = B.inst[slot];
+    BState* st = I.st;
+    if (!I.active || st->odone || st->done) return;
+    const long long chunk = blockIdx.x - I.chunk0;
+    double part[2] = {0.0, 0.0};
+    upd32_chunk(I, st, I.rounds, chunk, part);
+    double* const base = B.pf + I.chunk0;
+    if (!inst_arrive<2, RT>(part, base, B.nflat, chunk, I.nchunk, &st->tick_u, sh, &s_last)) return;
+    const double bn_in = __ldcg(&st->bn_in), tol_in = __ldcg(&st->tol_in), rho = __ldcg(&st->rho);
+    const long long total = __ldcg(&st->inner_total);
+    const int iter = __ldcg(&st->iter);
+    inst_total<2, RT, 8>(part, base, B.nflat, I.nchunk, &st->tick_u, sh);
     if (threadIdx.x != 0) return;
-    st->inner_total += 1;
-    st->pend = odd ? 0 : 1;
-    const double rel = __ddiv_rn(__dsqrt_rn(part[0]), st->bn_in);
+    st->inner_total = total + 1;
+    st->pend = iter & 1 ? 0 : 1;
+    const double rel = __ddiv_rn(__dsqrt_rn(part[0]), bn_in);
     if (!isfinite(rel) || !isfinite(part[1])) { st->inner_bad = 1; st->done = 1; return; }
-    if (rel < st->tol_in || st->iter + 1 >= B.max_inner) { st->done = 1; return; }
-    st->beta = __ddiv_rn(part[1], st->rho);
+    if (rel < tol_in || iter + 1 >= B.max_inner) { st->done = 1; return; }
+    st->beta = __ddiv_rn(part[1], rho);
     st->rho = part[1];
-    st->iter += 1;
+    st->iter = iter + 1;
 }
 
 // T += d (FP64) at the interior nodes, for the instances whose inner solve
