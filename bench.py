@@ -414,8 +414,8 @@ def main():
     # reductions); the graph's while body runs 4 iterations per pass, so a step
     # launches whole passes.  The atomic scatter adds p formation, zeroing and
     # the finishing pass to each operator.
-    # On small grids (N <= 88) the whole solve is one cooperative kernel.
-    if args.scatter == "colored" and N <= 88:
+    # Where the handle solves in one cooperative kernel, that is all of a step.
+    if g.coop_ctas:
         per_step, per_iter = 3, 0
     elif args.scatter == "colored":
         per_step, per_iter = 2 + 2 * (2 if detect else 1) + 2, 2

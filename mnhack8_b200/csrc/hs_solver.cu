@@ -392,7 +392,9 @@ const void* pcg_kernel(const hs_solver* h, bool runs) {
         default: return pcg_kernel_form<FORM_FAST>(nk, runs);
     }
 }
-// a run is one flat block up to N = 88; the waits take at most 2 RT tiles
+// the grids of the cooperative solve, if its CTAs fit the GPU: a run is one flat
+// block (UPD_SLOTS runs of RT*KF nodes: up to N = 71), and the waits take at most
+// 2 RT tiles
 bool coop_part(const Part& p) { return p.nflat <= UPD_SLOTS && p.nblk <= 2 * RT; }
 // the largest cooperative tile's shared memory
 size_t pcg_smem_most() {
