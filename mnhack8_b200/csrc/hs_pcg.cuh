@@ -46,7 +46,9 @@ __device__ __forceinline__ void xget(const XWord* w, double& v, unsigned long lo
 
 // Before the words of many CTAs are read, one thread waits for their count:
 // with 294 CTAs polling 294 words each, the polls themselves held the words up
-// (N=48: 10 us of an 18 us iteration).
+// (N=48: 10 us of an 18 us iteration).  A solve with the gate | without it, us:
+// N=16 (10 CTAs) 190 | 184, 24 (31) 280 | 279, 27 (43) 293 | 303, 29 (53) 310 | 344,
+// 36 (99) 370 | 513, 47 (288) 597 | 886, 71 (252) 1175 | 1450.
 constexpr int kGateCtas = 48;
 __device__ __forceinline__ void xgate(const unsigned* count, unsigned target) {
     if (threadIdx.x == 0) {
