@@ -136,13 +136,23 @@ BatchArgs batch_args(hs_batch* b) {
 // compact the live instances' tile and block ranges; grow the capacity (and
 // drop the graph) when they no longer fit; upload maps and descriptors
 hs_status upload(hs_batch* b) {
-    long long nt = 0, nf = 0, nc = 0;
-    for (auto& sl : b->slots) if (sl.used) { nt += sl.part.ntiles; nf += sl.part.nflat; nc += sl.desc.nchunk; }
+    long long nt = 0, nf = 0, nr = 0, nc = 0;
+    auto rounds_of = [](const hs_batch::Slot& sl) { return (sl.part.Nn + UR - 1) / UR; };
+    for (auto& sl : b->slots) if (sl.used) { nt += sl.part.ntiles; nf += sl.part.nflat; nr += rounds_of(sl); }
+    // rounds per block of the inner update, by all the instances' rounds
+    const int rounds = upd_rounds(nr);
+    for (auto& sl : b->slots)
+        if (sl.used) {
+            sl.desc.rounds = rounds;
+            sl.desc.nchunk = (rounds_of(sl) + rounds - 1) / rounds;
+            nc += sl.desc.nchunk;
+        }
     if (nt > b->cap_tiles || nf > b->cap_flat || nc > b->cap_chunk || !b->d_t2i.p) {
         b->cap_tiles = std::max<long long>({nt, 2 * b->cap_tiles, 1024});
         b->cap_flat = std::max<long long>({nf, 2 * b->cap_flat, 1024});
-        // a chunk holds several flat blocks, so there are at most as many
-        b->cap_chunk = std::max<long long>({nc, 2 * b->cap_chunk, 1024 / 4});
+        // with one or two rounds a block: kUpdBlocks and a ragged one per instance, so that
+        // fewer rounds, when instances leave, seldom need more (and a new graph)
+        b->cap_chunk = std::max<long long>({nc, 2 * b->cap_chunk, kUpdBlocks + 48});
         HS_CUDA(b->d_t2i.alloc(b->cap_tiles));
         HS_CUDA(b->d_f2i.alloc(b->cap_flat));
         HS_CUDA(b->d_c2i.alloc(b->cap_chunk));
@@ -467,8 +477,6 @@ hs_status batch_add_impl(hs_batch* b, int N, double dt, const double* k, const d
     sl.used = true; sl.N = N; sl.dt = dt; sl.steps_left = n_steps; sl.steps_done = 0;
     sl.part = batch_part(N, b->opt.tile_planes);
     d.part = sl.part;
-    d.rounds = upd_rounds(Nn);
-    d.nchunk = (Nn + (long long)d.rounds * UR - 1) / ((long long)d.rounds * UR);
     sl.mem = mem;
     sl.desc = d;
     b->dirty = true;

@@ -100,14 +100,14 @@ __device__ __forceinline__ bool fi_now(const BState* st, int vec) {
 struct BInst {
     Part part;                 // slab tiles and flat blocks of this instance
     long long tile0, flat0;    // first global tile / flat block
-    long long chunk0, nchunk;  // first global chunk of the inner update, and their number
+    long long chunk0, nchunk;  // first block of the inner update, and their number
     double dt;
     double cm[4], ck[4];       // wht eigen-constants / 8 of this grid
     float cmf[4], ckf[4];
     int active;
     int uniform;               // rho*c is one value: k32 holds k alone
     float rc32;                // and its value
-    int rounds;                // of the inner update's chunks (upd_rounds)
+    int rounds;                // of UR nodes that a block of it takes (upd_rounds)
     double* T;                 // solution (updated in place)
     double* b;                 // right-hand side M T_old
     double* y64;               // FP64 operator output
@@ -132,7 +132,7 @@ struct BatchArgs {
     const BInst* inst;
     const int* tile2inst;      // global tile -> instance slot (-1: none)
     const int* flat2inst;      // global flat block -> instance slot
-    const int* chunk2inst;     // global chunk -> instance slot
+    const int* chunk2inst;     // block of the inner update -> instance slot
     int n_inst, pad;
     long long ntiles, nflat, nchunk;   // capacity of the grids
     double* pa;                // apply partials: [q * ntiles + tile]
@@ -824,27 +824,35 @@ __global__ void __launch_bounds__(RT) kb_outer_final(BatchArgs B) {
 // r -= alpha Ap, z = r / diag; r.r and r.z; and at odd iterations d += alpha p
 // for the previous iteration and this one (the same two multiply-adds in the
 // same order; the previous p is still in the other buffer), which saves 4 of 32
-// bytes per node on average.  A block takes a chunk of consecutive nodes in rounds
-// of UR (UV groups of four per thread, a round's loads in flight together); the
-// last block of an instance to finish adds up its chunks' sums and does the inner
-// solve's scalar step (beta, convergence).
+// bytes per node on average.  The unit is a round of UR consecutive nodes (UV groups
+// of four per thread, their loads in flight together) with its own block tree and
+// partial sums, so an instance's bits do not depend on how rounds are dealt to
+// blocks.  The last block of an instance to finish adds up its rounds' sums and does
+// the inner solve's scalar step (beta, convergence).
 //
-// Rounds per chunk, by the grid alone (so that an instance has the same bits alone
-// and among others): one while that makes at most two blocks per SM (N <= 83), two
-// while all its blocks are resident at once (148 SMs of 4 blocks: N <= 133), else
-// four.  A small instance is bound by latency, and each further round is one more
-// chain of loads on a mostly idle GPU; a large one by the memory, and then by the
-// tree, fence and ticket that each block costs.  Device ms of 4 steps (B200) with
-// one | two | four rounds: 2 instances at N=48 5.20 | 5.40 | 5.83, 16 at N=64 23.9 |
-// 22.8 | 22.3, one at N=96 10.5 | 10.6 | 11.0, 16 at N=96 79.8 | 75.7 | 75.3, one at
-// N=128 15.5 | 14.7 | 15.1, 4 at N=128 56.4 | 54.0 | 52.7.
-constexpr int UV = 2, UR = RT * 4 * UV;
-inline int upd_rounds(long long Nn) {
-    return Nn <= 148ll * 2 * UR ? 1 : Nn <= 148ll * 4 * 2 * UR ? 2 : 4;
-}
-// the chunk's nodes; the thread's r.r and r.z into part
-__device__ __forceinline__ void upd32_chunk(const BInst& I, BState* st, int rounds, long long chunk, double (&part)[2]) {
-    const long long Nn = I.part.Nn;
+// Rounds per block, by the rounds of all instances: one while they are resident at
+// once (148 SMs of 4 blocks), two up to twice as many, else four.  Few are bound by
+// latency, and a further round in a block is one more chain of loads on a mostly idle
+// GPU; many by the memory, and then by the fence and ticket that each block costs.
+// Device ms of 4 steps (B200) with one | two | four rounds: 2 instances at N=16 2.45 |
+// 2.50 | 2.77, 2 at N=64 (268 rounds) 6.99 | 7.23 | 7.84, one at N=104 (566) 10.4 | 10.5 |
+// 11.2, one at N=112 (705) 14.0 | 13.3 | 13.8, 16 at N=48 (928) 9.08 | 8.74 | 9.28, 12 of
+// N=30..65 9.65 | 9.32 | 9.80, one at N=128 (1049) 14.5 | 14.1 | 14.7, one at N=140 (1369)
+// 20.0 | 19.8 | 18.9, 16 at N=96 78.4 | 75.1 | 74.7, 256 of N=17..92 315 | 296 | 288.
+constexpr int UV = 2, UR = RT * 4 * UV, UMAX = 4, kUpdBlocks = 148 * 4;
+inline int upd_rounds(long long all) { return all <= kUpdBlocks ? 1 : all <= 2 * kUpdBlocks ? 2 : UMAX; }
+__global__ void __launch_bounds__(RT, 4) kb_update32(BatchArgs B) {
+    __shared__ double sh[2][16];
+    __shared__ double shr[UMAX][2][RT / 32];
+    __shared__ unsigned s_last;
+    const int slot = B.chunk2inst[blockIdx.x];
+    if (slot < 0) return;
+    const BInst& I = B.inst[slot];
+    BState* st = I.st;
+    if (!I.active || st->odone || st->done) return;
+    const long long Nn = I.part.Nn, nround = (Nn + UR - 1) / UR;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, rounds = I.rounds;
+    const long long round0 = (blockIdx.x - I.chunk0) * rounds;
     const float alpha = (float)st->alpha;
     const bool odd = st->iter & 1;
     const float alpha_prev = odd ? (float)st->alpha_prev : 0.f;
@@ -863,7 +871,8 @@ __device__ __forceinline__ void upd32_chunk(const BInst& I, BState* st, int roun
     };
     float4 dv[UV], pv[UV], ov[UV], qv[UV], rv[UV], iv[UV];
     for (int ul = 0; ul < rounds; ++ul) {
-        const long long m0 = (chunk * rounds + ul) * UR + threadIdx.x * 4;
+        const long long m0 = (round0 + ul) * UR + threadIdx.x * 4;
+        double part[2] = {0.0, 0.0};
 #pragma unroll
         for (int u = 0; u < UV; ++u) {
             const long long m = m0 + u * (RT * 4);
@@ -895,25 +904,38 @@ __device__ __forceinline__ void upd32_chunk(const BInst& I, BState* st, int roun
             one(3, qv[u].w, rv[u].w, iv[u].w, zv.w);
             st4(I.r32, m, rv[u]); st4(I.z32, m, zv);
         }
+#pragma unroll
+        for (int off = 16; off >= 1; off >>= 1)
+#pragma unroll
+            for (int q = 0; q < 2; ++q) part[q] = dadd(part[q], __shfl_xor_sync(0xffffffffu, part[q], off));
+        if (lane == 0) { shr[ul][0][warp] = part[0]; shr[ul][1][warp] = part[1]; }
     }
-}
-__global__ void __launch_bounds__(RT, 4) kb_update32(BatchArgs B) {
-    __shared__ double sh[2][16];
-    __shared__ unsigned s_last;
-    const int slot = B.chunk2inst[blockIdx.x];
-    if (slot < 0) return;
-    const BInst& I = B.inst[slot];
-    BState* st = I.st;
-    if (!I.active || st->odone || st->done) return;
-    const long long chunk = blockIdx.x - I.chunk0;
-    double part[2] = {0.0, 0.0};
-    upd32_chunk(I, st, I.rounds, chunk, part);
-    double* const base = B.pf + I.chunk0;
-    if (!inst_arrive<2, RT>(part, base, B.nflat, chunk, I.nchunk, &st->tick_u, sh, &s_last)) return;
+    __syncthreads();
+    // the rounds' trees over the warp sums, two rounds of two quantities at a time; one
+    // partial per round (a quarter of the flat blocks), from the instance's flat0 on
+    double* const base = B.pf + I.flat0;
+    if (warp == 0) {
+        for (int h = 0; h < rounds; h += 2) {
+            const int ul = h + (lane >> 4), q = (lane >> 3) & 1;
+            double v = shr[ul][q][lane & 7];
+#pragma unroll
+            for (int off = 4; off >= 1; off >>= 1) v = dadd(v, __shfl_xor_sync(0xffffffffu, v, off));
+            if ((lane & 7) == 0 && ul < rounds && round0 + ul < nround) base[q * B.nflat + round0 + ul] = v;
+        }
+        __syncwarp();
+        if (lane == 0) {
+            __threadfence();
+            s_last = atomicAdd(&st->tick_u, 1u) == (unsigned)(I.nchunk - 1) ? 1u : 0u;
+        }
+    }
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
     const double bn_in = __ldcg(&st->bn_in), tol_in = __ldcg(&st->tol_in), rho = __ldcg(&st->rho);
     const long long total = __ldcg(&st->inner_total);
     const int iter = __ldcg(&st->iter);
-    inst_total<2, RT, 8>(part, base, B.nflat, I.nchunk, &st->tick_u, sh);
+    double part[2];
+    inst_total<2, RT, 8>(part, base, B.nflat, nround, &st->tick_u, sh);
     if (threadIdx.x != 0) return;
     st->inner_total = total + 1;
     st->pend = iter & 1 ? 0 : 1;
