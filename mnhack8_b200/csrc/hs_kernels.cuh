@@ -1226,8 +1226,9 @@ __global__ void k_step_begin(DevState* st, StepCtl c, double* T, unsigned* count
     if (c.flipG) T[c.gidx] = flipbit(T[c.gidx], c.bit);
 }
 __global__ void k_disarm_R(DevState* st) { st->fi_armR = 0; }
-__global__ void k_step_end(DevState* st, int* iters_out, double* d1_out, double* d1_last_out) {
+__global__ void k_step_end(DevState* st, int* iters_out, double* d1_out, double* d1_last_out, unsigned* gave_up) {
     st->fi_armR = 0; st->fi_vec = 0;
+    if (st->stuck) *gave_up = 1u;
     *iters_out = st->result;
     *d1_out = st->d1_step;
     if (d1_last_out) *d1_last_out = st->d1_last;

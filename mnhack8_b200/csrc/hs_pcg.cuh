@@ -144,7 +144,6 @@ struct PcgArgs {
     double* dparts;          // checksum partials: [3 sets][3][nblk]
     unsigned long long tag;  // this launch's first tag
     DevState* st;
-    unsigned* gave_up;       // page-locked host word: a wait gave up
     int with_rhs, nruns, d1;
     int fail_waits;          // every wait counts as given up (tests)
     ElemConsts ec;
@@ -398,7 +397,7 @@ __global__ void __launch_bounds__(ST, FORM == FORM_GAUSS ? 1 : 2) k_pcg(PcgArgs 
             st->d1_step = fmax(st->d1_step, rel);
         }
     };
-    auto stuck = [&]() { if (tid == 0) *a.gave_up = 1u; };
+    auto stuck = [&]() { if (tid == 0) st->stuck = 1; };        // (k_step_end tells the host)
 
     // ---- b = M T + dt F and Ap = A T -------------------------------------------------
     double2 cf[NK];

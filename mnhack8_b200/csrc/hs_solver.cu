@@ -448,7 +448,7 @@ hs_status launch_pcg(hs_solver* h, bool with_rhs) {
     a.with_rhs = with_rhs ? 1 : 0;
     a.nruns = update_runs(h);
     a.d1 = h->opt.detect != 0;
-    a.fail_waits = h->fail_waits; a.gave_up = h->gave_up.p;
+    a.fail_waits = h->fail_waits;
     a.ec = h->ec;
     void* args[] = {&a};
     HS_CUDA(cudaLaunchCooperativeKernel(h->coop_kernel, dim3(h->coop_grid), dim3(ST), args, pcg_smem(h->part.CX), h->s));
@@ -799,7 +799,7 @@ hs_status hs_apply(hs_solver* s, const double* x, double* y, double dt_eff, int 
         apply_projected(s, ROLE_RHS, x, y, dt_eff, d1, s->wM.p, nullptr, 0.0);
     else
         apply_projected(s, ROLE_X0, x, y, dt_eff, d1, s->wA.p, nullptr, 0.0);
-    k_step_end<<<1, 1, 0, s->s>>>(s->st.p, s->it_out.p, s->rec_out.p, s->rec_out.p + 6);
+    k_step_end<<<1, 1, 0, s->s>>>(s->st.p, s->it_out.p, s->rec_out.p, s->rec_out.p + 6, s->gave_up.p);
     HS_CUDA(cudaGetLastError());
     HS_CUDA(cudaStreamSynchronize(s->s));
     const hs_status st = check_waits(s);
@@ -878,7 +878,7 @@ hs_status enqueue_step(hs_solver* h, const hs_fi_spec* fi, int step, int reproje
     }
     if (reproject) k_set_boundary<<<grid_for(h->Nn, RT), RT, 0, h->s>>>(h->N, h->T.p, 0.0);
     if (e1) HS_CUDA(cudaEventRecord(e1, h->s));
-    k_step_end<<<1, 1, 0, h->s>>>(h->st.p, d_iters, d_d1, nullptr);
+    k_step_end<<<1, 1, 0, h->s>>>(h->st.p, d_iters, d_d1, nullptr, h->gave_up.p);
     HS_CUDA(cudaGetLastError());
     return HS_OK;
 }
@@ -951,7 +951,7 @@ hs_status hs_pcg(hs_solver* s, const double* b, double* x, int max_iter, double 
         st = pcg_direct(s, false);
         if (st != HS_OK) return st;
     }
-    k_step_end<<<1, 1, 0, s->s>>>(s->st.p, s->it_out.p, s->rec_out.p, nullptr);
+    k_step_end<<<1, 1, 0, s->s>>>(s->st.p, s->it_out.p, s->rec_out.p, nullptr, s->gave_up.p);
     HS_CUDA(cudaGetLastError());
     HS_CUDA(cudaMemcpyAsync(x, s->T.p, s->Nn * 8, cudaMemcpyDeviceToDevice, s->s));
     HS_CUDA(cudaStreamSynchronize(s->s));
